@@ -197,9 +197,11 @@ int siminf_gpu_run_solver_mssm(siminf_gpu_solver_args *args,
  * are drawn without knowledge of the state need it.
  *
  * heavy_rate: a tuning knob, not a semantic option -- nodes whose rate sum
- * at the start of a day reaches it are queued and simulated first, 32 to a
- * warp (results are identical either way); 0 takes the default (8), a
- * negative value turns the queue off.
+ * at the start of a day reaches it are queued and simulated first, each by
+ * a group of 8, 16 or 32 lanes (32 to a warp for models compiled from C
+ * code; results are identical either way); 0 takes the default (0.5 below
+ * 500,000 nodes in all replicates, 8 from there on and for compiled
+ * models), a negative value turns the queue off.
  *
  * two_pass: a tuning knob, not a semantic option -- each day first
  * finishes, one node per thread, every node whose day has no transition,
@@ -219,7 +221,7 @@ int siminf_gpu_run_solver_mssm(siminf_gpu_solver_args *args,
  */
 typedef struct siminf_gpu_options {
     int cap_transfers;
-    int heavy_rate;     /* rate sum from which a node is queued first (0 = default 8, < 0 = off) */
+    int heavy_rate;     /* rate sum from which a node is queued first (0 = default, < 0 = off) */
     int gdata_per_replicate;
     int two_pass;       /* > 0 on, < 0 off, 0 = on from 500,000 nodes (all replicates) */
     int max_node_day_transitions;   /* > 0: the bound; 0: 2^28 */
@@ -231,7 +233,8 @@ typedef struct siminf_gpu_options {
                          * registers a thread and fewer resident warps (see the autotuner) */
     int wave_block;     /* threads per block of the wavefront kernel: 128, 256 or 512 (0: 256) */
     int heavy_lanes;    /* lanes of a warp that take nodes of the heaviest class (rate sum
-                         * >= 16 x heavy_rate), 1..32 (0: 32) */
+                         * >= 16 x heavy_rate), 1..32 (0: 32), where no groups of lanes
+                         * step them (models compiled from C code) */
 } siminf_gpu_options;
 
 /* The default of siminf_gpu_options.max_node_day_transitions. */

@@ -1252,9 +1252,16 @@ static int plan_create_impl(const siminf_gpu_solver_args *a, const siminf_gpu_mo
     if (!rc) rc = dalloc(&s.queue_next, 6, own);
     if (!rc) rc = dalloc(&s.heavy_mark, (size_t) Ntot, own);
     /* heavy part of the work queue: threshold on the day-start rate sum
-     * (options, else SIMINF_HEAVY_RATE in the environment, 0 = off;
-     * default 8, the best of 2 to 128 on the 10^6-node SEIR workload) */
-    s.heavy_rate = 8.0;
+     * (options, else SIMINF_HEAVY_RATE in the environment, 0 = off).  Where
+     * groups of lanes step the heavy nodes, a small model lists nearly all
+     * its active nodes -- the chip has lanes to spare and a group's day is
+     * shorter than a lane's (SISe3 of 1,600 nodes, 730 days: 29.9 ms at 0.5,
+     * 46.5 at 8; SEIR of 100,000, 180 days: 27.1 against 28.9) -- and a
+     * large one, whose ordinary nodes fill the chip, lists the long chains
+     * only (SEIR of 10^6, 240 days: 108.7 ms at 8, 115.1 at 1).  Models
+     * without lane groups: 8, the best of 2 to 128 on the 10^6-node SEIR
+     * workload. */
+    s.heavy_rate = L->lane_groups && Ntot < 500000 ? 0.5 : 8.0;
     if (const char *ev = getenv("SIMINF_HEAVY_RATE"))
         s.heavy_rate = atof(ev);
     if (opt && opt->heavy_rate > 0)
@@ -2700,9 +2707,15 @@ int siminf_gpu_plan_tune(siminf_gpu_plan *p, void *cuda_stream, int probe_days,
      * against 2.76 s with 32) */
     if (!rc && best >= 0 && !p->s.aem)
         probe(r.heavy_rate[best], r.two_pass[best], 1, 256, 0);
-    if (!rc && best >= 0 && !p->s.aem && r.heavy_rate[best] > 0.0 && p->L->time_invariant &&
-        p->s.Nrep == 1 && !p->s.job_of)
+    if (p->L->lane_groups) {
+        /* heavy nodes have groups of lanes, whatever heavy_lanes says: the
+         * probe is of the plan's own threshold, where it is below all others */
+        if (!rc && best >= 0 && !p->s.aem && saved > 0.0 && saved < cand[1])
+            probe(saved, r.two_pass[best], r.ssa_variant[best], 256, 8);
+    } else if (!rc && best >= 0 && !p->s.aem && r.heavy_rate[best] > 0.0 &&
+               p->L->time_invariant && p->s.Nrep == 1 && !p->s.job_of) {
         probe(r.heavy_rate[best], r.two_pass[best], r.ssa_variant[best], 256, 8);
+    }
     /* stage 3: the wavefront block */
     if (!rc && best >= 0 && p->e2_count > 0) {
         const siminf_gpu_tune_result b = r;

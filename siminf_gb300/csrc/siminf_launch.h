@@ -15,6 +15,7 @@ struct Launchers {
     int Ngd;            /* gdata entries the model reads */
     bool pts_local;     /* post-time-step reads only its own node */
     bool time_invariant;    /* rates ignore t (the heavy part of the work queue applies) */
+    bool lane_groups;       /* heavy nodes are stepped by groups of lanes */
     cudaError_t (*init)(const DevState &s, double tt0, cudaStream_t st);
     cudaError_t (*horizon)(const DevState &s, const DayInfo *days, int ndays, cudaStream_t st);
     /* the first pass of a two-pass day (k_quick); ssa_e1 is the second */
@@ -53,7 +54,7 @@ const Launchers *launchers_for(const char *name);
  * the version with its own, which changes whenever the table or the device
  * state it passes changes layout. */
 #define SIMINF_MODEL_ABI \
-    (20261204 + (int) sizeof(siminf::DevState) + (int) sizeof(siminf::Launchers))
+    (20261205 + (int) sizeof(siminf::DevState) + (int) sizeof(siminf::Launchers))
 
 }  // namespace siminf
 

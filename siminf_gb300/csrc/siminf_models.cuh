@@ -35,6 +35,7 @@ struct ModelSIR {
     static constexpr int NGD = 0;  /* gdata entries read */
     static constexpr bool PTS_LOCAL = true;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
+    static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,
@@ -63,6 +64,7 @@ struct ModelSEIR {
     static constexpr int NGD = 0;  /* gdata entries read */
     static constexpr bool PTS_LOCAL = true;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
+    static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,
@@ -93,6 +95,7 @@ struct ModelSIS {
     static constexpr int NGD = 0;  /* gdata entries read */
     static constexpr bool PTS_LOCAL = true;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
+    static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,
@@ -149,6 +152,7 @@ struct ModelSISe {
     static constexpr int NGD = 8;  /* gdata entries read */
     static constexpr bool PTS_LOCAL = true;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
+    static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,
@@ -189,6 +193,7 @@ struct ModelSISe3 {
     static constexpr int NGD = 12;  /* gdata entries read */
     static constexpr bool PTS_LOCAL = true;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
+    static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,
@@ -262,6 +267,7 @@ struct ModelSISe_sp {
     static constexpr int NGD = 8;  /* gdata entries read */
     static constexpr bool PTS_LOCAL = false;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
+    static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,
@@ -301,6 +307,7 @@ struct ModelSISe3_sp {
     static constexpr int NGD = 12;  /* gdata entries read */
     static constexpr bool PTS_LOCAL = false;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
+    static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,
@@ -337,6 +344,7 @@ struct ModelSIRmparse {
     static constexpr int NGD = 2;  /* gdata entries read */
     static constexpr bool PTS_LOCAL = true;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
+    static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,
@@ -363,6 +371,7 @@ struct ModelSISePF {
     static constexpr int NGD = 2;  /* gdata entries read */
     static constexpr bool PTS_LOCAL = true;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
+    static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,

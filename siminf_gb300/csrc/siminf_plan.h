@@ -158,7 +158,8 @@ struct DevState {
     int wave_block;
     /* Lanes of a warp that take nodes of the heaviest class (1..32; 0:
      * 32): a warp that holds the day's longest chains shares its issue
-     * slots and FP64 pipe with fewer lanes. */
+     * slots and FP64 pipe with fewer lanes.  Read for models whose heavy
+     * nodes are not stepped by groups of lanes. */
     int heavy_lanes;
 
     /* Profiling: per day, the most transitions any node fired that day
