@@ -231,7 +231,7 @@ typedef struct siminf_gpu_options {
                          * before the plan returns */
     int ssa_variant;    /* SSA kernel register budget: 0 the model's default, 1 more
                          * registers a thread and fewer resident warps (see the autotuner) */
-    int wave_block;     /* threads per block of the wavefront kernel: 128, 256 or 512 (0: 256) */
+    int wave_block;     /* threads per block of the wavefront kernel: 128, 256 or 512 (0: 128) */
     int heavy_lanes;    /* lanes of a warp that take nodes of the heaviest class (rate sum
                          * >= 16 x heavy_rate), 1..32 (0: 32), where no groups of lanes
                          * step them (models compiled from C code) */

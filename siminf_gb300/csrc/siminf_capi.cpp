@@ -113,6 +113,41 @@ int upload(T **p, const T *src, size_t n, std::vector<void *> &owned, cudaStream
     return 0;
 }
 
+/* The first ncol columns of E on the device: the sparse matrix, and per
+ * column the compartments it selects from as a set (DevState::ecol). */
+int upload_E(DevState &s, const siminf_gpu_solver_args *a, int ncol, std::vector<void *> &owned,
+             cudaStream_t st)
+{
+    const int nnz = a->jcE[ncol];
+    std::vector<uint32_t> cols((size_t) std::max(ncol, 1), 0u);
+    for (int c = 0; c < ncol; c++) {
+        uint32_t rows = 0;
+        bool plain = true;
+        for (int k = a->jcE[c]; k < a->jcE[c + 1]; k++) {
+            const int row = a->irE[k];
+            plain = plain && row >= 0 && row < std::min(a->Nc, (int) MAX_NC) &&
+                    (k == a->jcE[c] || (row > a->irE[k - 1] && a->prE[k] == a->prE[k - 1]));
+            if (plain)
+                rows |= 1u << row;
+        }
+        cols[c] = plain ? rows | ECOL_PLAIN : 0u;
+    }
+    int *djc, *dir;
+    double *dpr;
+    uint32_t *dcol;
+    int rc = upload(&djc, a->jcE, (size_t) ncol + 1, owned, st);
+    if (!rc) rc = upload(&dir, a->irE, (size_t) nnz, owned, st);
+    if (!rc) rc = upload(&dpr, (const double *) a->prE, (size_t) nnz, owned, st);
+    if (!rc) rc = upload(&dcol, cols.data(), cols.size(), owned, st);
+    if (rc)
+        return rc;
+    s.jcE = djc;
+    s.irE = dir;
+    s.prE = dpr;
+    s.ecol = dcol;
+    return 0;
+}
+
 double ms_since(std::chrono::steady_clock::time_point t0)
 {
     return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -1192,16 +1227,7 @@ static int plan_create_impl(const siminf_gpu_solver_args *a, const siminf_gpu_mo
          * the events use (the struct carries no column counts; the
          * schedule scan found both). */
         const int maxsel = p->max_select, maxshift = p->max_shift;
-        const int ncolE = maxsel;
-        const int nnzE = a->jcE[ncolE];
-        int *dirE, *djcE;
-        double *dprE;
-        rc = upload(&djcE, a->jcE, (size_t) ncolE + 1, own, st);
-        if (!rc) rc = upload(&dirE, a->irE, (size_t) nnzE, own, st);
-        if (!rc) rc = upload(&dprE, (const double *) a->prE, (size_t) nnzE, own, st);
-        s.jcE = djcE;
-        s.irE = dirE;
-        s.prE = dprE;
+        rc = upload_E(s, a, maxsel, own, st);
         /* N is "defined" whenever the caller passes it (src/SimInf.c:302-305),
          * even if no event shifts. */
         s.hasN = a->N != nullptr;
@@ -1495,7 +1521,7 @@ static cudaError_t download_columns(const siminf_gpu_plan *p, const siminf_gpu_s
 
 /* The wavefronts of one day: offsets into d_e2 and event counts.  The
  * last ones, while each holds at most E2_TAIL_ITEMS events x replicates,
- * run together in one block (k_e2_tail), up to E2_TAIL_WAVES per launch;
+ * run together in one cluster (k_e2_tail), up to E2_TAIL_WAVES per launch;
  * the others, one launch each. */
 static cudaError_t launch_day_waves(const siminf_gpu_plan *p, const DevState &s,
                                     const long long *off, const long long *cnt, int nw, int d,
@@ -1513,9 +1539,12 @@ static cudaError_t launch_day_waves(const siminf_gpu_plan *p, const DevState &s,
     for (int w = t; w < nw && e == cudaSuccess; w += E2_TAIL_WAVES) {
         E2Tail tail;
         tail.n = std::min((int) E2_TAIL_WAVES, nw - w);
+        tail.wide = 0;
         for (int k = 0; k < tail.n; k++) {
             tail.off[k] = off[w + k];
             tail.count[k] = (int) cnt[w + k];
+            if (cnt[w + k] * (long long) s.Nrep > E2_BLOCK_ITEMS)
+                tail.wide = k + 1;
         }
         e = timed(kp, 2, st, [&] { return L->e2_tail(s, p->d_e2, tail, d, tt, st); });
     }
@@ -1767,19 +1796,14 @@ static cudaError_t launch_streamed(siminf_gpu_plan *p, DevState s, cudaStream_t 
             }
             /* E and N up to the largest select and shift seen so far */
             if (msel > p->max_select && a->jcE) {
-                int *djcE, *dirE;
-                double *dprE;
-                const int nnz = a->jcE[msel];
-                int rc = upload(&djcE, a->jcE, (size_t) msel + 1, p->owned, st);
-                if (!rc) rc = upload(&dirE, a->irE, (size_t) nnz, p->owned, st);
-                if (!rc) rc = upload(&dprE, (const double *) a->prE, (size_t) nnz, p->owned, st);
-                if (rc) {
+                if (upload_E(p->s, a, msel, p->owned, st)) {
                     e = cudaErrorMemoryAllocation;
                     break;
                 }
-                s.jcE = p->s.jcE = djcE;
-                s.irE = p->s.irE = dirE;
-                s.prE = p->s.prE = dprE;
+                s.jcE = p->s.jcE;
+                s.irE = p->s.irE;
+                s.prE = p->s.prE;
+                s.ecol = p->s.ecol;
                 p->max_select = msel;
             }
             if (mshift > p->max_shift && a->N) {
@@ -2291,19 +2315,14 @@ static cudaError_t launch_streamed_dev(siminf_gpu_plan *p, DevState s, cudaStrea
         }
         /* E and N up to the largest select and shift seen so far */
         if (pl.ch.max_select > p->max_select && a->jcE) {
-            int *djcE, *dirE;
-            double *dprE;
-            const int nnz = a->jcE[pl.ch.max_select];
-            int rc = upload(&djcE, a->jcE, (size_t) pl.ch.max_select + 1, p->owned, st);
-            if (!rc) rc = upload(&dirE, a->irE, (size_t) nnz, p->owned, st);
-            if (!rc) rc = upload(&dprE, (const double *) a->prE, (size_t) nnz, p->owned, st);
-            if (rc) {
+            if (upload_E(p->s, a, pl.ch.max_select, p->owned, st)) {
                 e = cudaErrorMemoryAllocation;
                 break;
             }
-            s.jcE = p->s.jcE = djcE;
-            s.irE = p->s.irE = dirE;
-            s.prE = p->s.prE = dprE;
+            s.jcE = p->s.jcE;
+            s.irE = p->s.irE;
+            s.prE = p->s.prE;
+            s.ecol = p->s.ecol;
             p->max_select = pl.ch.max_select;
         }
         if (pl.ch.max_shift > p->max_shift && a->N) {

@@ -1374,6 +1374,33 @@ __device__ __forceinline__ void load_u(const int *p, int (&u)[NC])
     }
 }
 
+/* load_u from L2, past the SM's own cache. */
+template <int NC>
+__device__ __forceinline__ void load_u_l2(const int *p, int (&u)[NC])
+{
+    if constexpr (NC % 4 == 0) {
+#pragma unroll
+        for (int c = 0; c < NC; c += 4) {
+            const int4 w = __ldcg(reinterpret_cast<const int4 *>(p + c));
+            u[c] = w.x;
+            u[c + 1] = w.y;
+            u[c + 2] = w.z;
+            u[c + 3] = w.w;
+        }
+    } else if constexpr (NC % 2 == 0) {
+#pragma unroll
+        for (int c = 0; c < NC; c += 2) {
+            const int2 w = __ldcg(reinterpret_cast<const int2 *>(p + c));
+            u[c] = w.x;
+            u[c + 1] = w.y;
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < NC; c++)
+            u[c] = __ldcg(p + c);
+    }
+}
+
 template <int NC>
 __device__ __forceinline__ void store_u(int *p, const int (&u)[NC])
 {
@@ -1876,22 +1903,23 @@ __global__ void __launch_bounds__(SSA_BLOCK, MINB) k_ssa_e1(DevState s, int day,
 /* One external transfer of one replicate (src/solvers/SimInf_solver.c:
  * 824-902): sample from the source, add to the destination (atomics: adds
  * into one destination commute within a wavefront), subtract from the
- * source (exclusive to this event within its wavefront). */
+ * source (exclusive to this event within its wavefront).  Any transfer;
+ * out of line behind e2_apply, which handles the common ones. */
 template <class M>
-__device__ __forceinline__ void e2_apply(const DevState &s, const E2Rec &e, int rep, int day,
-                                         double tt)
+__device__ __noinline__ void e2_apply_any(const DevState &s, const E2Rec &e, int rep, int day,
+                                          double tt)
 {
     constexpr int NC = M::NC;
     const long long gs = (long long) rep * s.Nn + e.src;
     const long long gd = (long long) rep * s.Nn + e.dst;
     int uu[NC], ind[NC];
     for (int c = 0; c < NC; c++)
-        uu[c] = s.u[gs * NC + c];
+        uu[c] = __ldcg(s.u + gs * NC + c);
     si_rng r;
     {
         uint64_t seed, sid;
         stream_key(s, gs, seed, sid);
-        si_rng_init(&r, seed, sid, s.ctr[gs]);
+        si_rng_init(&r, seed, sid, __ldcg((const unsigned long long *) s.ctr + gs));
     }
     int err = sample_select<NC>(s, uu, e.select, e.n, e.proportion, ind, &r);
     s.ctr[gs] = r.ctr;
@@ -1922,7 +1950,7 @@ __device__ __forceinline__ void e2_apply(const DevState &s, const E2Rec &e, int 
             }
             /* The source is exclusive to this event within the wave; a
              * self-transfer reads back its own atomic add. */
-            const int nv = s.u[gs * NC + jj] - ind[jj];
+            const int nv = __ldcg(s.u + gs * NC + jj) - ind[jj];
             s.u[gs * NC + jj] = nv;
             if (nv < 0) {
                 record_error(s, ERR_NEGATIVE_STATE, PHASE_E2, day, gs, -1, e.index, tt, 0);
@@ -1934,38 +1962,211 @@ __device__ __forceinline__ void e2_apply(const DevState &s, const E2Rec &e, int 
     s.update[gs] = 1;
 }
 
+/* Words of a node's stream held ready for a transfer's draws: the Philox
+ * blocks ctr >> 2 and the two after it, which every lane of a warp computes
+ * in step (drawn one block at a time when a lane runs out, some lane would
+ * be at a block's end at nearly every draw, and the warp would wait for a
+ * Philox block a draw).  A thread's words lie a block of threads apart in
+ * shared memory, one bank a lane. */
+enum { E2_WORDS = 12 };
+
+__device__ __forceinline__ uint32_t e2_word(const uint32_t *words, const si_rng &r, unsigned i)
+{
+    if (i < E2_WORDS)
+        return words[i * blockDim.x];
+    si_rng q = r;                       /* long samples: draw by draw from here on */
+    q.ctr = (r.ctr & ~3ull) + i;
+    q.have = 0;
+    return si_next_u32(&q);
+}
+
+/* The transfer of record e: a size given as a count, sampled from a plain
+ * column and moved unshifted to another node, runs here with the node's
+ * compartments in registers; everything else in e2_apply_any, with the same
+ * draws.  `words` is the thread's share of shared memory.  Bound: a wave's
+ * chain of dependent loads (record, state, then the atomics) and draws, and
+ * in waves that fill the chip instruction issue. */
 template <class M>
-__global__ void __launch_bounds__(512) k_e2_wave(DevState s, const E2Rec *ev, int count, int day,
+__device__ __forceinline__ void e2_apply(const DevState &s, const E2Rec &e, int rep, int day,
+                                         double tt, uint32_t *words)
+{
+    constexpr int NC = M::NC;
+    const long long gs = (long long) rep * s.Nn + e.src;
+    const long long gd = (long long) rep * s.Nn + e.dst;
+    int uu[NC], ind[NC];
+    load_u_l2<NC>(s.u + gs * NC, uu);
+    si_rng r;
+    {
+        uint64_t seed, sid;
+        stream_key(s, gs, seed, sid);
+        si_rng_init(&r, seed, sid, __ldcg((const unsigned long long *) s.ctr + gs));
+    }
+    const uint32_t col = s.ecol[e.select];
+    if (!(col & ECOL_PLAIN) || e.n <= 0 || e.shift >= 0 || e.src == e.dst) {
+        e2_apply_any<M>(s, e, rep, day, tt);
+        return;
+    }
+    const unsigned cols = col & ~ECOL_PLAIN;
+    int total = 0, kinds = 0;
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+        const bool in = (cols >> c) & 1u;
+        total += in ? uu[c] : 0;
+        kinds += in && uu[c] > 0;
+        ind[c] = 0;
+    }
+    int n = e.n;
+    if (s.cap && n > total)
+        n = total;
+    if (cols == 0 || n > total || n < 0) {
+        record_error(s, ERR_SAMPLE_SELECT, PHASE_E2, day, gs, -1, e.index, tt, 0);
+        return;
+    }
+    if (n > 0) {
+        if (n == total || kinds == 1) {
+            /* everyone, or n of the one kind there is */
+#pragma unroll
+            for (int c = 0; c < NC; c++)
+                if (((cols >> c) & 1u) && uu[c] > 0)
+                    ind[c] = n == total ? uu[c] : n;
+        } else {
+#pragma unroll
+            for (int b = 0; b < E2_WORDS / 4; b++) {
+                uint32_t w0, w1, w2, w3;
+                philox_block(r, (r.ctr >> 2) + b, w0, w1, w2, w3);
+                words[(4 * b) * blockDim.x] = w0;
+                words[(4 * b + 1) * blockDim.x] = w1;
+                words[(4 * b + 2) * blockDim.x] = w2;
+                words[(4 * b + 3) * blockDim.x] = w3;
+            }
+            /* sequential multivariate hypergeometric (SimInf_solver.c:
+             * 139-160); the urn of each compartment is si_hypergeometric's */
+            const unsigned first = (unsigned) r.ctr & 3u;
+            unsigned used = first;
+            int left = total, want = n;
+            for (unsigned rows = cols;; rows &= rows - 1) {
+                const int row = __ffs((int) rows) - 1;
+                int nk = uu[0];
+#pragma unroll
+                for (int c = 1; c < NC; c++)
+                    if (c == row)
+                        nk = uu[c];
+                const bool last = want == 0 || (rows & (rows - 1)) == 0;
+                int k = want;
+                if (!last) {
+                    const bool complement = 2 * (long long) want > left;
+                    const int t = complement ? left - want : want;
+                    unsigned a = (unsigned) nk, rem = (unsigned) left;
+                    k = 0;
+                    for (int i = 0; i < t && a > 0; i++) {
+                        if (a == rem) {
+                            k += t - i;
+                            break;
+                        }
+                        const uint32_t w = e2_word(words, r, used++);
+                        const bool take = (2 * (uint64_t) w + 1) * rem < ((uint64_t) a << 33);
+                        k += take;
+                        a -= take;
+                        rem--;
+                    }
+                    k = complement ? nk - k : k;
+                }
+#pragma unroll
+                for (int c = 0; c < NC; c++)
+                    if (c == row)
+                        ind[c] = k;
+                if (last)
+                    break;
+                left -= nk;
+                want -= k;
+            }
+            s.ctr[gs] = r.ctr + (used - first);
+        }
+        bool neg = false;
+#pragma unroll
+        for (int c = 0; c < NC; c++) {
+            if (ind[c])
+                neg |= atomicAdd(&s.u[gd * NC + c], ind[c]) + ind[c] < 0;
+            uu[c] -= ind[c];
+        }
+        store_u<NC>(s.u + gs * NC, uu);
+        if (neg) {
+            record_error(s, ERR_NEGATIVE_STATE, PHASE_E2, day, gs, -1, e.index, tt, 0);
+            return;
+        }
+    }
+    s.update[gd] = 1;
+    s.update[gs] = 1;
+}
+
+template <class M>
+__global__ void __launch_bounds__(512, 1) k_e2_wave(DevState s, const E2Rec *ev, int count, int day,
                                                  double tt)
 {
     const long long i = blockIdx.x * (long long) blockDim.x + threadIdx.x;
     if (i >= (long long) count * s.Nrep)
         return;
+    __shared__ uint32_t words[E2_WORDS * 512];
+    const int rep = s.Nrep == 1 ? 0 : (int) (i / count);
+    const E2Rec e = ev[i - (long long) rep * count];
     if (load_flag(s.err_day) < day || load_flag(s.err_day_pre_e2) <= day)
         return;
-    const int rep = (int) (i / count);
-    e2_apply<M>(s, ev[i - (long long) rep * count], rep, day, tt);
+    e2_apply<M>(s, e, rep, day, tt, words + threadIdx.x);
 }
 
-/* A day's last, small wavefronts in one block, in order, a barrier between
- * two (the block's writes before it are visible to the block after it):
- * one launch instead of one per wavefront.  Each holds at most
- * E2_TAIL_ITEMS = 1024 events x replicates, one per thread. */
-template <class M>
-__global__ void __launch_bounds__(1024) k_e2_tail(DevState s, const E2Rec *ev, E2Tail tail,
-                                                  int day, double tt)
+/* Every thread of the cluster has done its writes before any goes on, and
+ * sees them (release and acquire at cluster scope are the default). */
+__device__ __forceinline__ void cluster_barrier()
 {
-    if (load_flag(s.err_day) < day || load_flag(s.err_day_pre_e2) <= day)
+    asm volatile("barrier.cluster.arrive;\n\tbarrier.cluster.wait;" ::: "memory");
+}
+
+/* A day's last wavefronts in one launch, in order: the first `wide` of them
+ * by a cluster of E2_CLUSTER blocks with a cluster barrier between two, the
+ * smaller ones after them by the cluster's first block, where a block
+ * barrier is enough.  State is read from L2, where the other blocks' writes
+ * and the atomics are.  A wave on one SM is bound by that SM's issue slots
+ * from about 500 transfers on, which is where the second part begins; a
+ * wave that fills the cluster more than twice is better off on the whole
+ * chip.  With e2_apply's common path and draws in step, a day's transfers of
+ * SEIR, 10,000 nodes (9.7 waves): 79 us in three launches with a tail of one
+ * block, 47 in one launch; 10^6 nodes (15 waves): 187 us, then 138. */
+template <class M>
+__global__ void __launch_bounds__(E2_TAIL_BLOCK, 1) k_e2_tail(DevState s, const E2Rec *ev,
+                                                           E2Tail tail, int day, double tt)
+{
+    const bool stopped = load_flag(s.err_day) < day || load_flag(s.err_day_pre_e2) <= day;
+    if (stopped)
         return;                                     /* the same for every thread */
+    __shared__ uint32_t words[E2_WORDS * E2_TAIL_BLOCK];
+    const long long me = blockIdx.x * (long long) blockDim.x + threadIdx.x;
+    E2Rec e;
+    if (me < tail.count[0] * (long long) s.Nrep)
+        e = ev[tail.off[0] + (s.Nrep == 1 ? me : me % tail.count[0])];
     for (int w = 0; w < tail.n; w++) {
+        const bool wide = w < tail.wide;
+        if (!wide && blockIdx.x > 0)
+            return;
         const int count = tail.count[w];
         const E2Rec *wev = ev + tail.off[w];
         const long long items = (long long) count * s.Nrep;
-        for (long long i = threadIdx.x; i < items; i += blockDim.x) {
-            const int rep = (int) (i / count);
-            e2_apply<M>(s, wev[i - (long long) rep * count], rep, day, tt);
+        const long long step = wide ? (long long) gridDim.x * blockDim.x : blockDim.x;
+        for (long long i = me; i < items; i += step) {
+            const int rep = s.Nrep == 1 ? 0 : (int) (i / count);
+            if (i != me)
+                e = wev[i - (long long) rep * count];
+            e2_apply<M>(s, e, rep, day, tt, words + threadIdx.x);
         }
-        __syncthreads();
+        /* the thread's first record of the next wave, before the wait */
+        if (w + 1 < tail.n) {
+            const int nc = tail.count[w + 1];
+            if (me < nc * (long long) s.Nrep)
+                e = ev[tail.off[w + 1] + (s.Nrep == 1 ? me : me % nc)];
+        }
+        if (wide)
+            cluster_barrier();
+        else
+            __syncthreads();
     }
 }
 
@@ -2707,8 +2908,18 @@ struct Launch {
     static cudaError_t e2_tail(const DevState &s, const E2Rec *ev, const E2Tail &tail, int day,
                                double tt, cudaStream_t st)
     {
-        k_e2_tail<M><<<1, 1024, 0, st>>>(s, ev, tail, day, tt);
-        return cudaGetLastError();
+        cudaLaunchConfig_t cfg{};
+        cudaLaunchAttribute at{};
+        const unsigned blocks = tail.wide > 0 ? E2_CLUSTER : 1;
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(E2_TAIL_BLOCK);
+        cfg.stream = st;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = blocks;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, k_e2_tail<M>, s, ev, tail, day, tt);
     }
     static cudaError_t e2_wave(const DevState &s, const E2Rec *ev, int count, int day, double tt,
                                cudaStream_t st)
@@ -2716,7 +2927,7 @@ struct Launch {
         const long long n = (long long) count * s.Nrep;
         if (n == 0)
             return cudaSuccess;
-        const int b = (s.wave_block == 128 || s.wave_block == 512) ? s.wave_block : 256;
+        const int b = (s.wave_block == 256 || s.wave_block == 512) ? s.wave_block : 128;
         k_e2_wave<M><<<blocks_for(n, b), b, 0, st>>>(s, ev, count, day, tt);
         return cudaGetLastError();
     }

@@ -25,6 +25,7 @@
 namespace siminf {
 
 enum { MAX_NC = 16, MAX_NT = 32, MAX_ERR = 1024 };
+#define ECOL_PLAIN 0x80000000u
 
 /* k_ssa_e1 is a persistent grid fed by a per-day work queue of nodes: first
  * the heavy nodes (rate sum >= heavy_rate at the start of the day, listed by
@@ -57,12 +58,14 @@ struct E2Rec {          /* 32 bytes */
     double proportion;
 };
 
-/* A day's last, small wavefronts, run by one block (k_e2_tail): wave w
- * holds count[w] events from off[w] of the wave list (at most
- * E2_TAIL_WAVES waves of at most E2_TAIL_ITEMS events x replicates). */
-enum { E2_TAIL_WAVES = 32, E2_TAIL_ITEMS = 1024 };
+/* A day's last wavefronts, run by one launch of k_e2_tail: wave w holds
+ * count[w] events from off[w] of the wave list (at most E2_TAIL_WAVES waves
+ * of at most E2_TAIL_ITEMS events x replicates), the first `wide` of them
+ * with more than E2_BLOCK_ITEMS. */
+enum { E2_TAIL_WAVES = 32, E2_CLUSTER = 8, E2_TAIL_BLOCK = 512, E2_BLOCK_ITEMS = 512,
+       E2_TAIL_ITEMS = 2 * E2_CLUSTER * E2_TAIL_BLOCK };
 struct E2Tail {
-    int n;
+    int n, wide;
     int count[E2_TAIL_WAVES];
     long long off[E2_TAIL_WAVES];
 };
@@ -99,6 +102,10 @@ struct DevState {
     const uint32_t *Gmask;  /* Nt: bit k set if rate k is refreshed after transition j */
     const int *irE, *jcE;
     const double *prE;
+    /* per column of E: the set of compartments it selects from, with
+     * ECOL_PLAIN when the set says all that sampling needs (rows in
+     * ascending order, equal weights); 0 otherwise */
+    const uint32_t *ecol;
     const int *Nshift;      /* Nc x Nshift */
     int hasN;               /* the caller passed N */
     const double *ldata, *gdata;
@@ -153,7 +160,7 @@ struct DevState {
     /* Launch layout the autotuner picks: the SSA kernel's register budget
      * (0: the model's default, 1: more registers a thread and fewer
      * resident warps) and the external-transfer wave kernel's block size
-     * (128, 256 or 512; 0: 256). */
+     * (128, 256 or 512; 0: 128). */
     int ssa_variant;
     int wave_block;
     /* Lanes of a warp that take nodes of the heaviest class (1..32; 0:
