@@ -1269,6 +1269,7 @@ static int plan_create_impl(const siminf_gpu_solver_args *a, const siminf_gpu_mo
     s.crn_ctr = nullptr;
     if (!rc && a->crn == 1 && Nrep > 1 && a->solver == 0)
         rc = dalloc(&s.crn_ctr, (size_t) Ntot, own);
+    if (!rc && (!p->horizon || no_output)) rc = dalloc(&s.e1_next, (size_t) Ntot, own);
     if (!rc) rc = dalloc(&s.update, (size_t) Ntot, own);
     if (!rc) rc = dalloc(&s.err, (size_t) MAX_ERR, own);
     if (!rc) rc = dalloc(&s.err_count, 3, own);
@@ -1551,6 +1552,23 @@ static cudaError_t launch_day_waves(const siminf_gpu_plan *p, const DevState &s,
     return e;
 }
 
+/* Every node at the start of its E1 events (a run's list, or a chunk's). */
+__global__ void k_e1_start(DevState s)
+{
+    const long long g = blockIdx.x * (long long) blockDim.x + threadIdx.x;
+    if (g >= s.Ntot)
+        return;
+    const int node = (int) (s.Nrep == 1 ? g : g % s.Nn);
+    const int k = s.e1_ptr[node];
+    s.e1_next[g] = make_int2(k, k < s.e1_ptr[node + 1] ? s.e1[k].day : INT_MAX);
+}
+
+static cudaError_t e1_start(const DevState &s, cudaStream_t st)
+{
+    k_e1_start<<<(unsigned) ((s.Ntot + 255) / 256), 256, 0, st>>>(s);
+    return cudaGetLastError();
+}
+
 static cudaError_t launch_all(siminf_gpu_plan *p, DevState s, cudaStream_t st, KernelProfile *kp)
 {
     const Launchers *L = p->L;
@@ -1562,6 +1580,7 @@ static cudaError_t launch_all(siminf_gpu_plan *p, DevState s, cudaStream_t st, K
         return e;
     if (p->horizon)
         return timed(kp, 4, st, [&] { return L->horizon(s, p->d_days, ndays, st); });
+    e = timed(kp, 0, st, [&] { return e1_start(s, st); });
     for (int d = 0; d < ndays && e == cudaSuccess; d++) {
         const DayInfo &di = p->days[d];
         if (s.two_pass && !s.aem)
@@ -1920,6 +1939,8 @@ static cudaError_t launch_streamed(siminf_gpu_plan *p, DevState s, cudaStream_t 
             break;
         issued[c].store(1, std::memory_order_release);
         e = cudaStreamWaitEvent(st, copied[c], 0);
+        if (e == cudaSuccess && (c == 0 || sf))
+            e = e1_start(s, st);        /* the run's E1 list, or the chunk's */
         for (int d = d0; d < d1 && e == cudaSuccess; d++) {
             const DayInfo &di = p->days[d];
             if (s.two_pass && !s.aem)
@@ -2336,6 +2357,7 @@ static cudaError_t launch_streamed_dev(siminf_gpu_plan *p, DevState s, cudaStrea
         }
         s.e1 = pl.e1;
         s.e1_ptr = ring[c % E1_RING];
+        e = e1_start(s, st);
         const int d0 = c * CHUNK_DAYS, d1 = std::min(ndays, d0 + (int) CHUNK_DAYS);
         for (int d = d0; d < d1 && e == cudaSuccess; d++) {
             const int j = d - d0;

@@ -78,11 +78,27 @@ static __device__ __noinline__ void record_error(const DevState &s, int code, in
     }
 }
 
+/* Replicate and node of g, without the ~150 instructions of a 64-bit
+ * division where 32 bits or none will do. */
+__device__ __forceinline__ int rep_of(const DevState &s, long long g)
+{
+    if (s.Nrep == 1)
+        return 0;
+    return s.Ntot <= 0xFFFFFFFFll ? (int) ((unsigned) g / (unsigned) s.Nn) : (int) (g / s.Nn);
+}
+
+__device__ __forceinline__ int node_of(const DevState &s, long long g)
+{
+    return (int) (g - (long long) rep_of(s, g) * s.Nn);
+}
+
 __device__ __forceinline__ const double *gdata_of(const DevState &s, long long g)
 {
     if (s.job_of)
         return s.gdata + (size_t) s.job_of[g] * s.gdata_stride;
-    return s.gdata + (size_t) (g / s.Nn) * s.gdata_stride;
+    if (s.gdata_stride == 0)
+        return s.gdata;
+    return s.gdata + (size_t) rep_of(s, g) * s.gdata_stride;
 }
 
 /* Key of node g's stream: (seed, replicate * Nn + node) for one model, the
@@ -213,7 +229,7 @@ struct SsaLane {
  * which would never reach `next`). */
 template <class M>
 __device__ __forceinline__ bool ssa_begin(SsaLane<M> &ln, const si_rng &key, uint64_t c,
-                                          double next)
+                                          double next, const si_nl_tables *nl)
 {
     ln.fired = 0;
     ln.c = c;
@@ -232,7 +248,7 @@ __device__ __forceinline__ bool ssa_begin(SsaLane<M> &ln, const si_rng &key, uin
     uint32_t p0, p1, p2, p3;
     philox_block(key, c >> 2, p0, p1, p2, p3);
     philox_block(key, (c + 1) >> 2, ln.q0, ln.q1, ln.q2, ln.q3);
-    ln.L = si_neglog_u32(word_of(p0, p1, p2, p3, (uint32_t) c & 3u));
+    ln.L = si_neglog_u32_in(word_of(p0, p1, p2, p3, (uint32_t) c & 3u), nl);
     ln.U = si_u32_to_uniform_pos(word_of(ln.q0, ln.q1, ln.q2, ln.q3, (uint32_t) (c + 1) & 3u));
     if (!M::RATES_TIME_INVARIANT)
         ln.tau = si_div(ln.L, ln.sum);  /* ssa_step_ahead divides at each step */
@@ -395,7 +411,8 @@ template <class M, bool NEXT>
 __device__ __forceinline__ int ssa_step_spec(SsaLane<M> &ln, const si_rng &key, double L,
                                              double U, double next, const double *v,
                                              const double *ld, const double *gd, const int *sS,
-                                             const uint32_t *sG, unsigned max_fired)
+                                             const uint32_t *sG, unsigned max_fired,
+                                             const si_nl_tables *nl)
 {
     constexpr int NC = M::NC, NT = M::NT;
     int tau_special = 0;
@@ -450,7 +467,7 @@ __device__ __forceinline__ int ssa_step_spec(SsaLane<M> &ln, const si_rng &key, 
         const uint32_t ci = (uint32_t) c2 & 3u;
         const uint32_t wl = (ci == 3u) ? ln.q3 : word_of(n0, n1, n2, n3, ci);
         const uint32_t wu = word_of(n0, n1, n2, n3, (ci + 1u) & 3u);
-        L2 = si_neglog_u32_spec(wl, &redo);
+        L2 = si_neglog_u32_spec(wl, &redo, nl);
         U2 = si_u32_to_uniform_pos(wu);
     }
 
@@ -491,7 +508,7 @@ __device__ __forceinline__ int ssa_step_spec(SsaLane<M> &ln, const si_rng &key, 
  * uniform values.  The four -log(u) are independent chains of integer
  * operations that the compiler interleaves. */
 __device__ __forceinline__ void draw_four(const si_rng &key, uint64_t c, double (&L)[4],
-                                          double (&U)[4])
+                                          double (&U)[4], const si_nl_tables *nl)
 {
     uint32_t w[12];
     const uint64_t b = c >> 2;
@@ -506,13 +523,13 @@ __device__ __forceinline__ void draw_four(const si_rng &key, uint64_t c, double 
     int slow = 0;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        L[j] = si_neglog_u32_spec(x[2 * j], &slow);
+        L[j] = si_neglog_u32_spec(x[2 * j], &slow, nl);
         U[j] = si_u32_to_uniform_pos(x[2 * j + 1]);
     }
     if (slow) {
 #pragma unroll
         for (int j = 0; j < 4; j++)
-            L[j] = si_neglog_u32(x[2 * j]);
+            L[j] = si_neglog_u32_in(x[2 * j], nl);
     }
 }
 
@@ -526,17 +543,17 @@ template <class M>
 __device__ __forceinline__ void ssa_run_day(SsaLane<M> &ln, const si_rng &key, double next,
                                             const double *v, const double *ld, const double *gd,
                                             const int *sS, const uint32_t *sG,
-                                            unsigned max_fired)
+                                            unsigned max_fired, const si_nl_tables *nl)
 {
     for (;;) {
         double L[4], U[4];
-        draw_four(key, ln.c, L, U);
+        draw_four(key, ln.c, L, U, nl);
         int j = 0, st;
         double Lj, Uj;
         do {
             Lj = j == 0 ? L[0] : j == 1 ? L[1] : j == 2 ? L[2] : L[3];
             Uj = j == 0 ? U[0] : j == 1 ? U[1] : j == 2 ? U[2] : U[3];
-            st = ssa_step_spec<M, false>(ln, key, Lj, Uj, next, v, ld, gd, sS, sG, max_fired);
+            st = ssa_step_spec<M, false>(ln, key, Lj, Uj, next, v, ld, gd, sS, sG, max_fired, nl);
         } while (st == SSA_FIRED && ++j < 4);
         if (st == SSA_DAY_OVER)
             return;
@@ -560,7 +577,8 @@ __device__ __forceinline__ bool ssa_step_in_order(SsaLane<M> &ln, const si_rng &
                                                   double next, const double *v,
                                                   const double *ld, const double *gd,
                                                   const int *sS, const uint32_t *sG,
-                                                  unsigned max_fired)
+                                                  unsigned max_fired,
+                                                  const si_nl_tables *nl)
 {
     constexpr int NC = M::NC, NT = M::NT;
     const double tn = ln.tau + ln.t;
@@ -586,7 +604,7 @@ __device__ __forceinline__ bool ssa_step_in_order(SsaLane<M> &ln, const si_rng &
         ln.q1 = n1;
         ln.q2 = n2;
         ln.q3 = n3;
-        ln.L = si_neglog_u32(wl);
+        ln.L = si_neglog_u32_in(wl, nl);
         ln.U = si_u32_to_uniform_pos(wu);
     }
 
@@ -684,16 +702,17 @@ __device__ __forceinline__ bool ssa_step_in_order(SsaLane<M> &ln, const si_rng &
 template <class M>
 __device__ __forceinline__ bool ssa_step(SsaLane<M> &ln, const si_rng &key, double next,
                                          const double *v, const double *ld, const double *gd,
-                                         const int *sS, const uint32_t *sG, unsigned max_fired)
+                                         const int *sS, const uint32_t *sG, unsigned max_fired,
+                                                  const si_nl_tables *nl)
 {
     if constexpr (M::RATES_TIME_INVARIANT) {
         const int st = ssa_step_spec<M, true>(ln, key, ln.L, ln.U, next, v, ld, gd, sS, sG,
-                                              max_fired);
+                                              max_fired, nl);
         if (st != SSA_REDO)
             return st == SSA_DAY_OVER;
         return ssa_step_ahead<M>(ln, key, next, v, ld, gd, sS, sG, max_fired);
     } else {
-        return ssa_step_in_order<M>(ln, key, next, v, ld, gd, sS, sG, max_fired);
+        return ssa_step_in_order<M>(ln, key, next, v, ld, gd, sS, sG, max_fired, nl);
     }
 }
 
@@ -702,18 +721,19 @@ __device__ __forceinline__ bool ssa_step(SsaLane<M> &ln, const si_rng &key, doub
 template <class M>
 __device__ __forceinline__ unsigned ssa_day(SsaLane<M> &ln, si_rng &r, double next,
                                             const double *v, const double *ld, const double *gd,
-                                            const int *sS, const uint32_t *sG, unsigned max_fired)
+                                            const int *sS, const uint32_t *sG, unsigned max_fired,
+                                            const si_nl_tables *nl)
 {
-    if (!ssa_begin<M>(ln, r, r.ctr, next)) {
+    if (!ssa_begin<M>(ln, r, r.ctr, next, nl)) {
         /* two steps one at a time, then, for a node that is still going,
          * batches of four (a node with one transition or none in the day
          * computes no draws it does not use) */
         for (int n = 0;; n++) {
             if (M::RATES_TIME_INVARIANT && n == 2) {
-                ssa_run_day<M>(ln, r, next, v, ld, gd, sS, sG, max_fired);
+                ssa_run_day<M>(ln, r, next, v, ld, gd, sS, sG, max_fired, nl);
                 break;
             }
-            if (ssa_step<M>(ln, r, next, v, ld, gd, sS, sG, max_fired))
+            if (ssa_step<M>(ln, r, next, v, ld, gd, sS, sG, max_fired, nl))
                 break;
         }
     }
@@ -848,7 +868,8 @@ template <class M>
 __device__ __forceinline__ void ssa_day_group(SsaLane<M> &ln, const si_rng &key, const int W,
                                               bool live, double next, const double *v,
                                               const double *ld, const double *gd, const int *sS,
-                                              const uint32_t *sG, unsigned max_fired)
+                                              const uint32_t *sG, unsigned max_fired,
+                                              const si_nl_tables *nl)
 {
     constexpr int NC = M::NC, NT = M::NT;
     constexpr uint32_t ALL = NT == 32 ? 0xFFFFFFFFu : (1u << NT) - 1u;
@@ -886,7 +907,7 @@ __device__ __forceinline__ void ssa_day_group(SsaLane<M> &ln, const si_rng &key,
                 uint32_t r0, r1, r2;
                 philox_block(key, cw >> 2, r0, r1, r2, wl);
             }
-            L = si_neglog_u32(wl);
+            L = si_neglog_u32_in(wl, nl);
             U = si_u32_to_uniform_pos(word_of(p0, p1, p2, p3, (iw + 1u) & 3u));
         }
         int tr = select_transition<M>(ln.rate, U * ln.sum);
@@ -1031,7 +1052,7 @@ __device__ __forceinline__ void ssa_day_group(SsaLane<M> &ln, const si_rng &key,
                 /* the rest of the day on the exact path, by the first lane */
                 if (l == 0) {
                     const unsigned f = ln.fired;
-                    if (!ssa_begin<M>(ln, key, ln.c, next)) {
+                    if (!ssa_begin<M>(ln, key, ln.c, next, nl)) {
                         ln.fired = f;
                         while (!ssa_step_ahead<M>(ln, key, next, v, ld, gd, sS, sG, max_fired))
                             ;
@@ -1257,6 +1278,11 @@ __device__ int apply_e1(const DevState &s, int *uu, const E1Rec &e, si_rng *r)
     }
 }
 
+/* A node's place in its E1 events: the next one and its day (NO_E1 when
+ * there is none).  A day's events are found by looking at that day alone,
+ * where a bisection of the node's list was up to eight dependent loads. */
+enum { NO_E1 = INT_MAX };
+
 /* The E1 events of one node-day.  Inlined: a call would make the SSA
  * kernels save the registers live across it to local memory (spills),
  * while the samplers' code, after the SSA loop, runs only on the one
@@ -1267,50 +1293,42 @@ struct E1Out {
     int u[NC];
     uint64_t ctr;
     int err_code, err_event;
-    bool any;
+    int2 at;
 };
 
 template <int NC>
-__device__ __forceinline__ E1Out<NC> node_e1_apply(const DevState &s, E1Out<NC> o, si_rng r, int lo,
-                                                int end, int day)
+__device__ __forceinline__ E1Out<NC> node_e1_apply(const DevState &s, E1Out<NC> o, si_rng r, int end,
+                                                int day)
 {
-    for (int k = lo; k < end; k++) {
+    int k = o.at.x;
+    o.at.y = NO_E1;
+    for (; k < end; k++) {
         const E1Rec e = s.e1[k];
-        if (e.day != day)
+        if (e.day != day) {
+            o.at.y = e.day;
             break;
+        }
         const int err = apply_e1<NC>(s, o.u, e, &r);
-        o.any = true;
         if (err) {
             o.err_code = err;
             o.err_event = e.index;
             break;
         }
     }
+    o.at.x = k;
     o.ctr = r.ctr;
     return o;
 }
 
 /* The node's E1 events of `day` (src/solvers/SimInf_solver.c:658-822), in
- * array order, applied to u with draws from r.  Returns true when an event
- * was applied (the node is then flagged for a rate refresh).  A node's
- * events are stored in day order: the day's first is found by bisection. */
+ * array order, applied to u with draws from r; `at`, the node's place in
+ * its events, moves past them.  Returns true when an event was applied (the
+ * node is then flagged for a rate refresh). */
 template <int NC>
-__device__ __forceinline__ bool node_e1(const DevState &s, int (&u)[NC], int node, int day,
-                                        si_rng &r, long long g, double tt, int &err_code,
-                                        int &err_event)
+__device__ __forceinline__ bool node_e1(const DevState &s, int (&u)[NC], int2 &at, int node, int day,
+                                        si_rng &r, int &err_code, int &err_event)
 {
-    int lo = s.e1_ptr[node], hi = s.e1_ptr[node + 1];
-    if (lo == hi)
-        return false;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if (s.e1[mid].day < day)
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    const int end = s.e1_ptr[node + 1];
-    if (lo >= end || s.e1[lo].day != day)
+    if (at.y != day)
         return false;
     E1Out<NC> o;
 #pragma unroll
@@ -1319,30 +1337,30 @@ __device__ __forceinline__ bool node_e1(const DevState &s, int (&u)[NC], int nod
     o.ctr = r.ctr;
     o.err_code = 0;
     o.err_event = -1;
-    o.any = false;
-    o = node_e1_apply<NC>(s, o, r, lo, end, day);
+    o.at = at;
+    o = node_e1_apply<NC>(s, o, r, s.e1_ptr[node + 1], day);
 #pragma unroll
     for (int c = 0; c < NC; c++)
         u[c] = o.u[c];
     r.ctr = o.ctr;
     r.have = 0;
+    at = o.at;
     if (o.err_code) {
         err_code = o.err_code;
         err_event = o.err_event;
     }
-    return o.any;
+    return true;
 }
 
 /* node_e1 as a call, for k_horizon with models of at most two
  * compartments: inlined, its samplers take the registers the one-node-a-
  * thread loop keeps live and 12 bytes spill; called, they do not (and the
- * call is made only for a node that has E1 events at all). */
+ * call is made only on a day with events). */
 template <int NC>
-__device__ __noinline__ bool node_e1_call(const DevState &s, int (&u)[NC], int node, int day,
-                                          si_rng &r, long long g, double tt, int &err_code,
-                                          int &err_event)
+__device__ __noinline__ bool node_e1_call(const DevState &s, int (&u)[NC], int2 &at, int node,
+                                          int day, si_rng &r, int &err_code, int &err_event)
 {
-    return node_e1<NC>(s, u, node, day, r, g, tt, err_code, err_event);
+    return node_e1<NC>(s, u, at, node, day, r, err_code, err_event);
 }
 
 /* The NC compartments of one node, loaded or stored with 16-byte (NC a
@@ -1483,6 +1501,18 @@ __device__ __forceinline__ void load_model_smem(const DevState &s, int *sS, uint
     __syncthreads();
 }
 
+/* The tables of -log(u) in shared memory, for kernels whose every step
+ * looks them up: a kernel starts with a cold L1, and two of the lookups
+ * depend on one another.  Followed by a barrier of the caller's. */
+__device__ __forceinline__ void load_nl_smem(si_nl_tables &nl)
+{
+    static_assert(sizeof(si_nl_tables) % sizeof(uint4) == 0, "copied 16 bytes at a time");
+    const uint4 *from = reinterpret_cast<const uint4 *>(&si_nl_dev);
+    uint4 *to = reinterpret_cast<uint4 *>(&nl);
+    for (unsigned i = threadIdx.x; i < sizeof(si_nl_tables) / sizeof(uint4); i += blockDim.x)
+        to[i] = from[i];
+}
+
 /* ------------------------------------------------------------------ */
 /* Kernels.                                                              */
 /* ------------------------------------------------------------------ */
@@ -1502,31 +1532,34 @@ __device__ __forceinline__ int heavy_class(const DevState &s, double sum)
     return si_dge(sum, 16.0 * s.heavy_rate) ? 0 : si_dge(sum, 4.0 * s.heavy_rate) ? 1 : 2;
 }
 
-/* Warp-wide (every lane of the warp calls it): lanes with cls >= 0 append
- * their node to heavy list cls of `day`, with one atomic per class present
- * in the warp; a list that is full takes nothing more. */
-__device__ __forceinline__ void push_heavy_warp(const DevState &s, long long g, int cls, int day)
+/* Block-wide (every thread calls it): nodes with a class >= 0 join that
+ * class's heavy list of `day`, up to two nodes a thread.  Places within the
+ * block are taken in shared memory; one thread a class then takes the
+ * block's places in the list, the three side by side (class after class and
+ * warp by warp, six pushes of two round trips to L2 each, k_pts_store took
+ * 14.3 us a day at 10,000 nodes, and now takes 10.5).  A list that is full
+ * takes nothing more. */
+__device__ __forceinline__ void push_heavy(const DevState &s, long long g1, int cls1, long long g2,
+                                           int cls2, int day)
 {
-    const unsigned FULL = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int c = 0; c < HEAVY_CLASSES; c++) {
-        const unsigned m = __ballot_sync(FULL, cls == c);
-        if (!m)
-            continue;
-        const int q = (day & 1) * HEAVY_CLASSES + c;
-        const int leader = __ffs(m) - 1;
-        int base = MAX_HEAVY;
-        if (lane == leader && load_flag(&s.heavy_count[q]) < MAX_HEAVY)
-            base = atomicAdd(&s.heavy_count[q], __popc(m));
-        base = __shfl_sync(FULL, base, leader);
-        if (cls == c) {
-            const int slot = base + __popc(m & ((1u << lane) - 1u));
-            if (slot < MAX_HEAVY) {
-                s.heavy_list[q * MAX_HEAVY + slot] = (int) g;
-                s.heavy_mark[g] = day + 1;
-            }
-        }
+    __shared__ int count[HEAVY_CLASSES], base[HEAVY_CLASSES];
+    if (threadIdx.x < HEAVY_CLASSES)
+        count[threadIdx.x] = 0;
+    __syncthreads();
+    const int at1 = cls1 >= 0 ? atomicAdd(&count[cls1], 1) : 0;
+    const int at2 = cls2 >= 0 ? atomicAdd(&count[cls2], 1) : 0;
+    __syncthreads();
+    const int q = (day & 1) * HEAVY_CLASSES;
+    if (threadIdx.x < HEAVY_CLASSES && count[threadIdx.x] > 0)
+        base[threadIdx.x] = atomicAdd(&s.heavy_count[q + threadIdx.x], count[threadIdx.x]);
+    __syncthreads();
+    if (cls1 >= 0 && base[cls1] + at1 < MAX_HEAVY) {
+        s.heavy_list[(q + cls1) * MAX_HEAVY + base[cls1] + at1] = (int) g1;
+        s.heavy_mark[g1] = day + 1;
+    }
+    if (cls2 >= 0 && base[cls2] + at2 < MAX_HEAVY) {
+        s.heavy_list[(q + cls2) * MAX_HEAVY + base[cls2] + at2] = (int) g2;
+        s.heavy_mark[g2] = day + 1;
     }
 }
 
@@ -1537,7 +1570,7 @@ __device__ __forceinline__ int init_node(const DevState &s, long long g, double 
     constexpr int NC = M::NC, NT = M::NT, ND = M::ND;
     if (s.pf_days)
         tt0 = s.pf_days[(size_t) *s.pf_interval * s.pf_days_stride].tt;
-    const int node = (int) (g % s.Nn);
+    const int node = node_of(s, g);
     int u[NC];
     load_u<NC>(s.u + g * NC, u);
     const double *v = s.vA + g * ND;
@@ -1568,14 +1601,14 @@ __global__ void k_init(DevState s, double tt0)
     int cls = -1;
     if (g < s.Ntot)
         cls = init_node<M>(s, g, tt0);
-    push_heavy_warp(s, g, cls, 0);
+    push_heavy(s, g, cls, 0, -1, 0);
 }
 
 /* The end of a node's day: its E1 events (or its SSA error) and the state
  * written back. */
 template <class M>
 __device__ __forceinline__ void node_finish(const DevState &s, SsaLane<M> &ln, si_rng &r,
-                                            long long g, int day, double tt,
+                                            long long g, int2 at, int day, double tt,
                                             unsigned long long &fired)
 {
     constexpr int NC = M::NC, NT = M::NT;
@@ -1596,9 +1629,10 @@ __device__ __forceinline__ void node_finish(const DevState &s, SsaLane<M> &ln, s
         record_error(s, ln.err, PHASE_SSA, day, g, ln.err_tr, -1, ln.err_t, ln.err_rate);
     } else {
         int e_code = 0, e_idx = -1;
-        const bool upd = node_e1<NC>(s, ln.u, (int) (g % s.Nn), day, r, g, tt, e_code, e_idx);
-        if (upd)
+        if (node_e1<NC>(s, ln.u, at, node_of(s, g), day, r, e_code, e_idx)) {
             s.update[g] = 1;
+            s.e1_next[g] = at;
+        }
         if (e_code)
             record_error(s, e_code, PHASE_E1, day, g, -1, e_idx, tt, 0);
     }
@@ -1685,17 +1719,17 @@ __global__ void __launch_bounds__(256) k_quick(DevState s, int day, double tt, d
             if (err) {
                 record_error(s, err, PHASE_SSA, day, g, -1, -1, t, sum);
             } else {
-                const int node = (int) (g % s.Nn);
-                if (s.e1_ptr[node] != s.e1_ptr[node + 1]) {
+                int2 at = s.e1_next[g];
+                if (at.y == day) {
                     int u[NC];
                     load_u<NC>(s.u + g * NC, u);
                     r.ctr = c;
                     r.have = 0;
                     int e_code = 0, e_idx = -1;
-                    if (node_e1<NC>(s, u, node, day, r, g, tt, e_code, e_idx)) {
-                        s.update[g] = 1;
-                        store_u<NC>(s.u + g * NC, u);
-                    }
+                    node_e1<NC>(s, u, at, node_of(s, g), day, r, e_code, e_idx);
+                    s.update[g] = 1;
+                    s.e1_next[g] = at;
+                    store_u<NC>(s.u + g * NC, u);
                     if (e_code)
                         record_error(s, e_code, PHASE_E1, day, g, -1, e_idx, tt, 0);
                     c = r.ctr;
@@ -1742,8 +1776,20 @@ __global__ void __launch_bounds__(SSA_BLOCK, MINB) k_ssa_e1(DevState s, int day,
     constexpr int NC = M::NC, NT = M::NT, ND = M::ND;
     __shared__ int sS[NT * NC];
     __shared__ uint32_t sG[NT];
-    load_model_smem<M>(s, sS, sG);
+    __shared__ __align__(16) si_nl_tables nl;
     const int par = day & 1, npar = (day + 1) & 1;
+    /* the loads that everything waits for, all in flight at once */
+    const int err_day = load_flag(s.err_day);
+    int n[HEAVY_CLASSES];
+#pragma unroll
+    for (int c = 0; c < HEAVY_CLASSES; c++)
+        n[c] = s.heavy_count[par * HEAVY_CLASSES + c];
+    /* the ordinary part: every node in index order, or on two-pass days
+     * the nodes k_quick listed */
+    const unsigned long long Ntot = s.two_pass ? s.queue_next[4 + par]
+                                               : (unsigned long long) s.Ntot;
+    load_nl_smem(nl);
+    load_model_smem<M>(s, sS, sG);
     if (blockIdx.x == 0 && threadIdx.x < HEAVY_CLASSES)
         s.heavy_count[npar * HEAVY_CLASSES + threadIdx.x] = 0;  /* filled by this day's pts */
     if (blockIdx.x == 0 && threadIdx.x < 2)
@@ -1751,27 +1797,27 @@ __global__ void __launch_bounds__(SSA_BLOCK, MINB) k_ssa_e1(DevState s, int day,
     if (blockIdx.x == 0 && threadIdx.x == 2)
         s.queue_next[4 + npar] = 0;                     /* filled by the next k_quick */
     unsigned long long fired = 0;
-    if (load_flag(s.err_day) < day) {
+    if (err_day < day) {
         add_fired(s, fired);
         return;
     }
-    int n[HEAVY_CLASSES];
     unsigned long long H = 0;
 #pragma unroll
     for (int c = 0; c < HEAVY_CLASSES; c++) {
-        n[c] = min(s.heavy_count[par * HEAVY_CLASSES + c], (int) MAX_HEAVY);
+        n[c] = min(n[c], (int) MAX_HEAVY);
         H += (unsigned long long) n[c];
     }
-    /* the ordinary part: every node in index order, or on two-pass days
-     * the nodes k_quick listed */
-    const unsigned long long Ntot = s.two_pass ? s.queue_next[4 + par]
-                                               : (unsigned long long) s.Ntot;
     const int lane = threadIdx.x & 31;
     const unsigned FULL = 0xFFFFFFFFu;
+    /* each warp's first heavy entry is its own number, so that only later
+     * ones cost an atomic's round trip */
+    const unsigned nwarp = gridDim.x * (SSA_BLOCK / 32);
+    const unsigned warp = blockIdx.x * (SSA_BLOCK / 32) + threadIdx.x / 32;
 
     SsaLane<M> ln;
     si_rng r;
     long long g = -1;
+    int2 e1 = make_int2(0, NO_E1);      /* the node's place in its E1 events */
     bool alive = true, need = true, done = false, heavy = false;
     bool heavy_left = H > 0;         /* warp-uniform: the heavy part may have entries */
     const double *v = nullptr, *ld = nullptr, *gd = nullptr;
@@ -1779,36 +1825,35 @@ __global__ void __launch_bounds__(SSA_BLOCK, MINB) k_ssa_e1(DevState s, int day,
         /* the heavy part: an entry is one node of the first class for the
          * whole warp, two of the second for 16 lanes each, or four of the
          * third for 8 */
-        const unsigned long long end0 = n[0], end1 = end0 + (unsigned long long) (n[1] + 1) / 2;
-        const unsigned long long items = end1 + (unsigned long long) (n[2] + 3) / 4;
-        while (heavy_left) {
-            unsigned long long at = 0;
-            if (lane == 0)
-                at = atomicAdd(&s.queue_next[par * 2], 1ull);
-            at = __shfl_sync(FULL, at, 0);
-            if (at >= items)
-                break;
+        const unsigned end0 = n[0], end1 = end0 + (n[1] + 1) / 2, items = end1 + (n[2] + 3) / 4;
+        unsigned at = warp;
+        while (at < items) {
             const int c = at < end0 ? 0 : at < end1 ? 1 : 2;
-            const int W = 32 >> c;
-            const int idx = ((int) (at - (c == 0 ? 0 : c == 1 ? end0 : end1)) << c) + lane / W;
+            const int idx = ((int) (at - (c == 0 ? 0 : c == 1 ? end0 : end1)) << c) +
+                            (lane >> (5 - c));
             bool live = idx < n[c];
             g = s.heavy_list[(par * HEAVY_CLASSES + c) * MAX_HEAVY + (live ? idx : 0)];
             live = live && !job_over(s, g, day);
             load_node<M>(s, g, ln, r);
             ln.c = s.crn_ctr ? s.crn_ctr[g] : s.ctr[g];
-            ssa_day_group<M>(ln, r, W, live, next, s.vA + g * ND,
-                             s.ldata + (size_t) (g % s.Nn) * s.Nld, gdata_of(s, g), sS, sG,
-                             s.max_fired);
-            if (live && (lane & (W - 1)) == 0)
-                node_finish<M>(s, ln, r, g, day, tt, fired);
+            e1 = s.e1_next[g];
+            ssa_day_group<M>(ln, r, 32 >> c, live, next, s.vA + g * ND,
+                             s.ldata + (size_t) node_of(s, g) * s.Nld, gdata_of(s, g), sS, sG,
+                             s.max_fired, &nl);
+            if (live && (lane & ((32 >> c) - 1)) == 0)
+                node_finish<M>(s, ln, r, g, e1, day, tt, fired);
             __syncwarp();
+            if (nwarp >= items)
+                break;
+            if (lane == 0)
+                at = nwarp + (unsigned) atomicAdd(&s.queue_next[par * 2], 1ull);
+            at = __shfl_sync(FULL, at, 0);
         }
         heavy_left = false;
     }
     /* lanes of a warp that take ordinary nodes: a day of few nodes is spread
      * over all warps of the grid, so that a warp steps fewer chains whose
      * branches exclude one another */
-    const unsigned long long nwarp = (unsigned long long) gridDim.x * (SSA_BLOCK / 32);
     const unsigned lanes =
         s.two_pass ? 32u : (unsigned) min(32ull, (Ntot + nwarp - 1) / nwarp);
     alive = lane < (int) max(lanes, 1u) || heavy_left;
@@ -1865,9 +1910,10 @@ __global__ void __launch_bounds__(SSA_BLOCK, MINB) k_ssa_e1(DevState s, int day,
                 heavy = from_heavy;
                 load_node<M>(s, g, ln, r);
                 v = s.vA + g * ND;
-                ld = s.ldata + (size_t) (g % s.Nn) * s.Nld;
+                ld = s.ldata + (size_t) node_of(s, g) * s.Nld;
                 gd = gdata_of(s, g);
-                done = ssa_begin<M>(ln, r, s.crn_ctr ? s.crn_ctr[g] : s.ctr[g], next);
+                e1 = s.e1_next[g];
+                done = ssa_begin<M>(ln, r, s.crn_ctr ? s.crn_ctr[g] : s.ctr[g], next, &nl);
                 need = false;
             }
         }
@@ -1875,7 +1921,7 @@ __global__ void __launch_bounds__(SSA_BLOCK, MINB) k_ssa_e1(DevState s, int day,
             break;
         if (alive && !need) {
             if (done) {
-                node_finish<M>(s, ln, r, g, day, tt, fired);
+                node_finish<M>(s, ln, r, g, e1, day, tt, fired);
                 need = true;
                 heavy = false;
             } else {
@@ -1884,14 +1930,14 @@ __global__ void __launch_bounds__(SSA_BLOCK, MINB) k_ssa_e1(DevState s, int day,
                  * do not read t */
                 if constexpr (M::RATES_TIME_INVARIANT) {
                     if (heavy) {
-                        ssa_run_day<M>(ln, r, next, v, ld, gd, sS, sG, s.max_fired);
+                        ssa_run_day<M>(ln, r, next, v, ld, gd, sS, sG, s.max_fired, &nl);
                         done = true;
                     } else {
-                        done = ssa_step<M>(ln, r, next, v, ld, gd, sS, sG, s.max_fired);
+                        done = ssa_step<M>(ln, r, next, v, ld, gd, sS, sG, s.max_fired, &nl);
                     }
                 } else {
                     do
-                        done = ssa_step<M>(ln, r, next, v, ld, gd, sS, sG, s.max_fired);
+                        done = ssa_step<M>(ln, r, next, v, ld, gd, sS, sG, s.max_fired, &nl);
                     while (heavy && !done);
                 }
             }
@@ -2205,7 +2251,7 @@ __device__ __forceinline__ int pts_node(const DevState &s, long long g, int day,
                                         int c0, int c1, const double *v_in, double *v_out)
 {
     constexpr int NC = M::NC, ND = M::ND;
-    const int rep = (int) (g / s.Nn), node = (int) (g % s.Nn);
+    const int rep = rep_of(s, g), node = node_of(s, g);
     int u[NC];
     load_u<NC>(s.u + g * NC, u);
     const double *vi = v_in + g * ND;
@@ -2236,7 +2282,7 @@ __device__ __forceinline__ int refresh_node(const DevState &s, long long g, int 
                                             const double *v_out)
 {
     constexpr int NC = M::NC, NT = M::NT, ND = M::ND;
-    const int node = (int) (g % s.Nn);
+    const int node = node_of(s, g);
     int u[NC];
     load_u<NC>(s.u + g * NC, u);
     const double *vo = v_out + g * ND;
@@ -2281,15 +2327,14 @@ __global__ void __launch_bounds__(256) k_pts_store(DevState s, int day, double t
             cls = -1;
         }
     }
-    push_heavy_warp(s, g, cls, day + 1);
     __syncthreads();
-    long long gr = -1;
+    long long gr = 0;
     int cls2 = -1;
     if (threadIdx.x < nlisted) {
         gr = g0 + listed[threadIdx.x];
         cls2 = refresh_node<M>(s, gr, day, tt, v_out);
     }
-    push_heavy_warp(s, gr, cls2, day + 1);
+    push_heavy(s, g, cls, gr, cls2, day + 1);
 }
 
 /* ------------------------------------------------------------------ */
@@ -2365,7 +2410,7 @@ __global__ void k_aem_init(DevState s, double tt0)
     int cls = -1;
     if (g < s.Ntot)
         cls = aem_init_node<M>(s, g, tt0);
-    push_heavy_warp(s, g, cls, 0);
+    push_heavy(s, g, cls, 0, -1, 0);
 }
 
 /* k_aem_init for one node; returns its heavy class on day 0 (from the sum
@@ -2374,7 +2419,7 @@ template <class M>
 __device__ __forceinline__ int aem_init_node(const DevState &s, long long g, double tt0)
 {
     constexpr int NC = M::NC, NT = M::NT, ND = M::ND;
-    const int node = (int) (g % s.Nn);
+    const int node = node_of(s, g);
     int u[NC];
     load_u<NC>(s.u + g * NC, u);
     const double *v = s.vA + g * ND;
@@ -2501,8 +2546,11 @@ __device__ __forceinline__ void aem_finish(const DevState &s, AemNode<M> &a, lon
         record_error(s, a.err, PHASE_SSA, day, g, a.err_tr, -1, a.err_t, a.err_rate);
     } else {
         int e_code = 0, e_idx = -1;
-        if (node_e1<NC>(s, a.u, (int) (g % s.Nn), day, r, g, tt, e_code, e_idx))
+        int2 at = s.e1_next[g];
+        if (node_e1<NC>(s, a.u, at, node_of(s, g), day, r, e_code, e_idx)) {
             s.update[g] = 1;
+            s.e1_next[g] = at;
+        }
         if (e_code)
             record_error(s, e_code, PHASE_E1, day, g, -1, e_idx, tt, 0);
     }
@@ -2598,7 +2646,7 @@ __global__ void __launch_bounds__(SSA_BLOCK, M::NT <= 4 ? 4 : 3) k_aem_day(DevSt
             if (cand >= 0) {
                 g = cand;
                 heavy = from_heavy;
-                const int node = (int) (g % s.Nn);
+                const int node = node_of(s, g);
                 load_u<NC>(s.u + g * NC, a.u);
 #pragma unroll
                 for (int j = 0; j < NT; j++) {
@@ -2656,7 +2704,7 @@ __global__ void __launch_bounds__(256) k_aem_pts(DevState s, int day, double tt,
     int cls = -1;
     if (g < s.Ntot && load_flag(s.err_day) >= day)
         cls = aem_pts_node<M>(s, g, day, tt, c0, c1, v_in, v_out);
-    push_heavy_warp(s, g, cls, day + 1);
+    push_heavy(s, g, cls, 0, -1, day + 1);
 }
 
 /* k_aem_pts for one node; returns its heavy class on the next day. */
@@ -2665,7 +2713,7 @@ __device__ __forceinline__ int aem_pts_node(const DevState &s, long long g, int 
                                             int c0, int c1, const double *v_in, double *v_out)
 {
     constexpr int NC = M::NC, NT = M::NT, ND = M::ND;
-    const int rep = (int) (g / s.Nn), node = (int) (g % s.Nn);
+    const int rep = rep_of(s, g), node = node_of(s, g);
     AemNode<M> a;
     load_u<NC>(s.u + g * NC, a.u);
     const double *vi = v_in + g * ND;
@@ -2729,11 +2777,13 @@ __global__ void __launch_bounds__(256, M::NT <= 4 ? 2 : 1) k_horizon(DevState s,
     constexpr int NC = M::NC, NT = M::NT, ND = M::ND;
     __shared__ int sS[NT * NC];
     __shared__ uint32_t sG[NT];
+    __shared__ __align__(16) si_nl_tables nl;
+    load_nl_smem(nl);
     load_model_smem<M>(s, sS, sG);
     const long long g = blockIdx.x * (long long) blockDim.x + threadIdx.x;
     unsigned long long fired = 0;
     if (g < s.Ntot) {
-        const int rep = (int) (g / s.Nn), node = (int) (g % s.Nn);
+        const int rep = rep_of(s, g), node = node_of(s, g);
         SsaLane<M> ln;
         load_u<NC>(s.u + g * NC, ln.u);
 #pragma unroll
@@ -2759,6 +2809,9 @@ __global__ void __launch_bounds__(256, M::NT <= 4 ? 2 : 1) k_horizon(DevState s,
         double *v = s.vA + g * ND, *vn = s.vB + g * ND;
         const double *ld = s.ldata + (size_t) node * s.Nld;
         const double *gd = gdata_of(s, g);
+        int2 at;
+        at.x = s.e1_ptr[node];
+        at.y = at.x < s.e1_ptr[node + 1] ? s.e1[at.x].day : NO_E1;
         for (int d = 0; d < ndays; d++) {
             if (load_flag(s.err_day) < d)
                 break;
@@ -2767,7 +2820,7 @@ __global__ void __launch_bounds__(256, M::NT <= 4 ? 2 : 1) k_horizon(DevState s,
             ln.err_tr = -1;
             ln.err_t = 0.0;
             ln.err_rate = 0.0;
-            fired += ssa_day<M>(ln, r, di.next, v, ld, gd, sS, sG, s.max_fired);
+            fired += ssa_day<M>(ln, r, di.next, v, ld, gd, sS, sG, s.max_fired, &nl);
             if (ln.err) {
                 record_error(s, ln.err, PHASE_SSA, d, g, ln.err_tr, -1, ln.err_t, ln.err_rate);
                 break;
@@ -2782,10 +2835,10 @@ __global__ void __launch_bounds__(256, M::NT <= 4 ? 2 : 1) k_horizon(DevState s,
             }
             bool upd = false;
             if constexpr (NC <= 2) {
-                if (s.e1_ptr[node] != s.e1_ptr[node + 1])
-                    upd = node_e1_call<NC>(s, ln.u, node, d, r, g, di.tt, e_code, e_idx);
+                if (at.y == d)
+                    upd = node_e1_call<NC>(s, ln.u, at, node, d, r, e_code, e_idx);
             } else {
-                upd = node_e1<NC>(s, ln.u, node, d, r, g, di.tt, e_code, e_idx);
+                upd = node_e1<NC>(s, ln.u, at, node, d, r, e_code, e_idx);
             }
             if (s.crn_ctr) {
                 const uint64_t t = r.ctr;   /* back to the SSA's */
@@ -2902,8 +2955,15 @@ struct Launch {
     }
     static cudaError_t ssa_e1(const DevState &s, int day, double tt, double next, cudaStream_t st)
     {
-        return s.ssa_variant == 1 ? ssa_e1_with<SSA_MINB1>(s, day, tt, next, st)
-                                  : ssa_e1_with<SSA_MINB0>(s, day, tt, next, st);
+        /* the larger register budget also where its warps have at most two
+         * nodes each: a model that small has no use for more warps (SISe3,
+         * 1,600 nodes: 100 bytes a thread spilled under the smaller one) */
+        const bool small = model_rates_total<M>::value &&
+                           (long long) blocks_for(s.Ntot, SSA_BLOCK / 16) <=
+                               ssa_resident_blocks<SSA_MINB1>();
+        return s.ssa_variant == 1 || small
+                   ? ssa_e1_with<SSA_MINB1>(s, day, tt, next, st)
+                   : ssa_e1_with<SSA_MINB0>(s, day, tt, next, st);
     }
     static cudaError_t e2_tail(const DevState &s, const E2Rec *ev, const E2Tail &tail, int day,
                                double tt, cudaStream_t st)
@@ -2934,7 +2994,10 @@ struct Launch {
     static cudaError_t pts_store(const DevState &s, int day, double tt, int c0, int c1,
                                  const double *v_in, double *v_out, cudaStream_t st)
     {
-        k_pts_store<M><<<blocks_for(s.Ntot, 256), 256, 0, st>>>(s, day, tt, c0, c1, v_in, v_out);
+        /* small models in small blocks, over more SMs: the FP64 pipe takes a
+         * warp instruction in 64 cycles, and two warps would share one */
+        const int b = s.Ntot <= 65536 ? 64 : 256;
+        k_pts_store<M><<<blocks_for(s.Ntot, b), b, 0, st>>>(s, day, tt, c0, c1, v_in, v_out);
         return cudaGetLastError();
     }
     static cudaError_t aem_init(const DevState &s, double tt0, cudaStream_t st)

@@ -21,6 +21,7 @@
 #define SIMINF_PLAN_H
 
 #include <stdint.h>
+#include <vector_types.h>
 
 namespace siminf {
 
@@ -126,6 +127,9 @@ struct DevState {
     /* events */
     const int *e1_ptr;
     const E1Rec *e1;
+    /* per g: the next of the node's E1 events (an index of e1) and its day
+     * (INT_MAX: none left); set whenever e1 is, kept by the kernels */
+    int2 *e1_next;
 
     /* outputs: dense or sparse (pattern on the device) */
     int *U;

@@ -431,22 +431,27 @@ SI_HD double si_log(double x)
 /* -log of a 32-bit uniform, for the SSA's exponential waiting time.  */
 /* ---------------------------------------------------------------- */
 
-static const uint32_t si_nl_r1_host[128] = SI_NL_R1_INIT;
-static const uint64_t si_nl_l1_host[128] = SI_NL_L1_INIT;
-static const uint32_t si_nl_r2_host[256] = SI_NL_R2_INIT;
-static const int64_t si_nl_l2_host[256] = SI_NL_L2_INIT;
-static const uint64_t si_nl_kln2_host[34][2] = SI_NL_KLN2_INIT;
+/* The tables of si_neglog_u32: one copy for host code, one in device global
+ * memory; a kernel whose every step looks them up keeps its own in shared
+ * memory (si_neglog_u32_in). */
+typedef struct si_nl_tables {
+    uint64_t l1[128];
+    int64_t l2[256];
+    uint64_t kln2[34][2];
+    uint32_t r1[128];
+    uint32_t r2[256];
+} si_nl_tables;
+
+#define SI_NL_TABLES_INIT                                                                       \
+    {SI_NL_L1_INIT, SI_NL_L2_INIT, SI_NL_KLN2_INIT, SI_NL_R1_INIT, SI_NL_R2_INIT}
+static const si_nl_tables si_nl_host = SI_NL_TABLES_INIT;
 #ifdef __CUDACC__
-static __device__ const uint32_t si_nl_r1_dev[128] = SI_NL_R1_INIT;
-static __device__ const uint64_t si_nl_l1_dev[128] = SI_NL_L1_INIT;
-static __device__ const uint32_t si_nl_r2_dev[256] = SI_NL_R2_INIT;
-static __device__ const int64_t si_nl_l2_dev[256] = SI_NL_L2_INIT;
-static __device__ const uint64_t si_nl_kln2_dev[34][2] = SI_NL_KLN2_INIT;
+static __device__ __align__(16) const si_nl_tables si_nl_dev = SI_NL_TABLES_INIT;
 #endif
 #ifdef __CUDA_ARCH__
-#  define SI_NL(tab) si_nl_##tab##_dev
+#  define SI_NL_GLOBAL (&si_nl_dev)
 #else
-#  define SI_NL(tab) si_nl_##tab##_host
+#  define SI_NL_GLOBAL (&si_nl_host)
 #endif
 
 SI_HD int si_clz32(uint32_t x)
@@ -472,7 +477,7 @@ SI_HD uint64_t si_mulw(uint32_t a, uint32_t b)
  * 2^-61.  That is within one ulp for u <= 1 - 2^-8 (0.97 ulp at worst over
  * all 2^32 words); si_neglog_u32 sends larger u (probability 2^-8) to
  * si_log.  Integer-only: the same bits on every host and device. */
-SI_HD double si_neglog_u32_tab(uint32_t w)
+SI_HD double si_neglog_u32_tab(uint32_t w, const si_nl_tables *nl)
 {
     const uint64_t x = 2 * (uint64_t) w + 1;
     int k;
@@ -486,10 +491,10 @@ SI_HD double si_neglog_u32_tab(uint32_t w)
         M = (uint64_t) xl << (32 - k);
     }
     const int j1 = (int) ((M >> 25) & 127);
-    const uint64_t M1 = M * (uint64_t) SI_NL(r1)[j1];          /* (m r1) * 2^42 */
+    const uint64_t M1 = M * (uint64_t) nl->r1[j1];          /* (m r1) * 2^42 */
     const int64_t Z1 = (int64_t) M1 - ((int64_t) 1 << 42);    /* |Z1| < 2^35 */
     const int j2 = (int) (((uint64_t) (Z1 + ((int64_t) 1 << 35)) >> 28) & 255);
-    const uint64_t M2 = M1 * (uint64_t) SI_NL(r2)[j2];         /* (m r1 r2) * 2^58 */
+    const uint64_t M2 = M1 * (uint64_t) nl->r2[j2];         /* (m r1 r2) * 2^58 */
     const int64_t Z2 = (int64_t) M2 - ((int64_t) 1 << 58);    /* z * 2^58, |.| < 2^43.5 */
 
     /* ln(1 + z) * 2^64 = z - z^2/2 + z^3/3 - z^4/4 */
@@ -508,11 +513,11 @@ SI_HD double si_neglog_u32_tab(uint32_t w)
     const int64_t ln1p = z1t - (int64_t) t2 + s3 - (int64_t) t4;
 
     /* (33 - k) ln 2 - L1 - L2 - ln(1+z) in Q64.64 */
-    uint64_t hi = SI_NL(kln2)[33 - k][0], lo = SI_NL(kln2)[33 - k][1];
-    const uint64_t l1 = SI_NL(l1)[j1];
+    uint64_t hi = nl->kln2[33 - k][0], lo = nl->kln2[33 - k][1];
+    const uint64_t l1 = nl->l1[j1];
     hi -= (lo < l1);
     lo -= l1;
-    const int64_t l2 = SI_NL(l2)[j2] + ln1p;                 /* |.| < 2^58 */
+    const int64_t l2 = nl->l2[j2] + ln1p;                 /* |.| < 2^58 */
     const uint64_t l2u = (uint64_t) l2;
     const uint64_t l2h = (uint64_t) (l2 >> 63);              /* sign extension */
     hi -= l2h + (lo < l2u);
@@ -537,11 +542,11 @@ SI_HD double si_neglog_u32_tab(uint32_t w)
 /* si_neglog_u32 for a speculative step: the table value in straight-line
  * code, with *slow set when w is one of the words (probability 2^-8) that
  * si_neglog_u32 hands to si_log instead. */
-SI_HD double si_neglog_u32_spec(uint32_t w, int *slow)
+SI_HD double si_neglog_u32_spec(uint32_t w, int *slow, const si_nl_tables *nl)
 {
     const uint64_t x = 2 * (uint64_t) w + 1;
     *slow |= x >= ((uint64_t) 1 << 33) - ((uint64_t) 1 << 25);
-    return si_neglog_u32_tab(w);
+    return si_neglog_u32_tab(w, nl);
 }
 
 #ifdef __CUDACC__
@@ -554,7 +559,7 @@ static __device__ __noinline__ double si_neglog_slow(uint32_t w)
 }
 #endif
 
-SI_HD double si_neglog_u32(uint32_t w)
+SI_HD double si_neglog_u32_in(uint32_t w, const si_nl_tables *nl)
 {
     const uint64_t x = 2 * (uint64_t) w + 1;
     if (x >= ((uint64_t) 1 << 33) - ((uint64_t) 1 << 25)) {
@@ -564,7 +569,12 @@ SI_HD double si_neglog_u32(uint32_t w)
         return -si_log(si_u32_to_uniform_pos(w));
 #endif
     }
-    return si_neglog_u32_tab(w);
+    return si_neglog_u32_tab(w, nl);
+}
+
+SI_HD double si_neglog_u32(uint32_t w)
+{
+    return si_neglog_u32_in(w, SI_NL_GLOBAL);
 }
 
 /* ---------------------------------------------------------------- */
