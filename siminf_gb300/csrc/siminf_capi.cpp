@@ -3067,7 +3067,7 @@ static int pf_session_create(const siminf_gpu_solver_args *a1, const siminf_gpu_
     p->days_cap = p->ndays;
     const cudaStream_t pst = p->stream;
     rc = upload(&ss->d_lfact, lfact.data(), lfact.size(), p->owned, pst);
-    if (!rc) rc = dalloc(&ss->d_w, (size_t) Np, p->owned);
+    if (!rc) rc = dalloc(&ss->d_w, (size_t) 3 * Np, p->owned);
     if (!rc) rc = dalloc(&ss->d_anc, (size_t) Np, p->owned);
     if (!rc) rc = dalloc(&ss->d_anc_out, (size_t) Np * pf->n_obs, p->owned);
     if (!rc) rc = upload(&ss->d_obs, pf->obs, (size_t) pf->n_obs * Nn, p->owned, pst);

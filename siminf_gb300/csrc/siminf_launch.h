@@ -35,7 +35,8 @@ struct Launchers {
                            double tt, cudaStream_t st);
 };
 
-/* Particle-filter kernels (model independent). */
+/* Particle-filter kernels (model independent); pf_finalize's w has room for
+ * three values a particle. */
 cudaError_t pf_weights(const int *U, int tlen, int Nn, int Nc, int Np, const int *obs_row,
                        int obs_c, const double *lfact, int tablen, double logp, double logq,
                        double *w, cudaStream_t st, const int *interval = nullptr);
