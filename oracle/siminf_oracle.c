@@ -1278,6 +1278,17 @@ void oracle_neglog_u32(const uint32_t *w, double *out, int64_t n)
         out[i] = si_neglog_u32(w[i]);
 }
 
+/* The integer-pipe operations: a * n, (double) n and (int) a. */
+void oracle_exact_ops(const double *a, const int *n, double *product, double *conv, int *trunc,
+                      int64_t count)
+{
+    for (int64_t i = 0; i < count; i++) {
+        product[i] = si_mul_i(a[i], n[i]);
+        conv[i] = si_i2d(n[i]);
+        trunc[i] = si_d2i(a[i]);
+    }
+}
+
 void oracle_philox(uint32_t *ctr4, uint32_t k0, uint32_t k1)
 {
     si_philox4x32_10(&ctr4[0], &ctr4[1], &ctr4[2], &ctr4[3], k0, k1);

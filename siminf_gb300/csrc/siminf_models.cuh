@@ -12,9 +12,10 @@
  * The expressions, and their evaluation order, are those of the reference
  * model files (cited per model); the library is compiled with -fmad=false so
  * that no multiply-add is fused and every double rounds as it does in the
- * reference's C.  Three exact substitutions move work off GB300's slow FP64
+ * reference's C.  Four exact substitutions move work off GB300's slow FP64
  * pipe without changing a single bit of any result: int -> double
- * conversions are built from integer bits (si_i2d), a double sum of integer
+ * conversions are built from integer bits (si_i2d), a product with a count
+ * is rounded from its integer digits (si_mul_i), a double sum of integer
  * counts that stays below 2^53 is formed as an integer sum and converted once
  * (every partial sum is exact either way), and divisions use si_div, an
  * IEEE round-to-nearest division on the integer pipes.  rate() takes a
@@ -42,14 +43,12 @@ struct ModelSIR {
                                                   double t, DC &dc)
     {
         if (k == 0) {
-            const double S_n = si_i2d(u[0]);
-            const double I_n = si_i2d(u[1]);
             const long long n = (long long) u[0] + u[1] + u[2];     /* S_n + I_n + u[R] */
             /* the population divides every call: its reciprocal is cached */
-            const double q = si_div_cached(ldata[0] * S_n * I_n, si_l2d(n > 0 ? n : 1), &dc);
+            const double q = si_div_cached(si_mul_i(si_mul_i(ldata[0], u[0]), u[1]), si_l2d(n > 0 ? n : 1), &dc);
             return n > 0 ? q : 0.0;
         }
-        return ldata[1] * si_i2d(u[1]);
+        return si_mul_i(ldata[1], u[1]);
     }
     __device__ __forceinline__ static int pts(double *, const int *, const double *,
                                               const double *, const double *, int, double)
@@ -71,16 +70,14 @@ struct ModelSEIR {
                                                   double t, DC &dc)
     {
         if (k == 0) {
-            const double S_n = si_i2d(u[0]);
-            const double I_n = si_i2d(u[2]);
             const long long n = (long long) u[0] + u[1] + u[2] + u[3];  /* S_n + u[E] + I_n + u[R] */
             /* the population divides every call: its reciprocal is cached */
-            const double q = si_div_cached(ldata[0] * S_n * I_n, si_l2d(n > 0 ? n : 1), &dc);
+            const double q = si_div_cached(si_mul_i(si_mul_i(ldata[0], u[0]), u[2]), si_l2d(n > 0 ? n : 1), &dc);
             return n > 0 ? q : 0.0;
         }
         if (k == 1)
-            return ldata[1] * si_i2d(u[1]);
-        return ldata[2] * si_i2d(u[2]);
+            return si_mul_i(ldata[1], u[1]);
+        return si_mul_i(ldata[2], u[2]);
     }
     __device__ __forceinline__ static int pts(double *, const int *, const double *,
                                               const double *, const double *, int, double)
@@ -102,14 +99,12 @@ struct ModelSIS {
                                                   double t, DC &dc)
     {
         if (k == 0) {
-            const double S_n = si_i2d(u[0]);
-            const double I_n = si_i2d(u[1]);
             const long long n = (long long) u[0] + u[1];               /* S_n + I_n */
             /* the population divides every call: its reciprocal is cached */
-            const double q = si_div_cached(ldata[0] * S_n * I_n, si_l2d(n > 0 ? n : 1), &dc);
+            const double q = si_div_cached(si_mul_i(si_mul_i(ldata[0], u[0]), u[1]), si_l2d(n > 0 ? n : 1), &dc);
             return n > 0 ? q : 0.0;
         }
-        return ldata[1] * si_i2d(u[1]);
+        return si_mul_i(ldata[1], u[1]);
     }
     __device__ __forceinline__ static int pts(double *, const int *, const double *,
                                               const double *, const double *, int, double)
@@ -159,29 +154,28 @@ struct ModelSISe {
                                                   double t, DC &dc)
     {
         if (k == 0)
-            return gdata[0] * v[0] * si_i2d(u[0]);
-        return gdata[1] * si_i2d(u[1]);
+            return si_mul_i(gdata[0] * v[0], u[0]);
+        return si_mul_i(gdata[1], u[1]);
     }
     __device__ __forceinline__ static int pts(double *v_new, const int *u, const double *v,
                                               const double *ldata, const double *gdata,
                                               int node, double t)
     {
-        const int day = (int) t % 365;
-        const double I_n = u[1];
-        const double n = u[0] + I_n;
+        const int day = si_d2i(t) % 365;
+        const long long n = (long long) u[0] + u[1];
         const double phi = v[0];
-        v_new[0] = forward_euler_linear_decay(phi, day, (int) ldata[0], (int) ldata[1],
-                                              (int) ldata[2], (int) ldata[3], gdata[3],
+        v_new[0] = forward_euler_linear_decay(phi, day, si_d2i(ldata[0]), si_d2i(ldata[1]),
+                                              si_d2i(ldata[2]), si_d2i(ldata[3]), gdata[3],
                                               gdata[4], gdata[5], gdata[6]);
-        if (n > 0.0)
-            v_new[0] += gdata[2] * I_n / n + gdata[7];
+        if (n > 0)
+            v_new[0] += si_div(si_mul_i(gdata[2], u[1]), si_l2d(n)) + gdata[7];
         else
             v_new[0] += gdata[7];
         if (!isfinite(v_new[0]))
             return -7;          /* SIMINF_ERR_V_IS_NOT_FINITE */
-        if (v_new[0] < 0.0)
+        if (si_bad_rate(v_new[0]))
             return -10;         /* SIMINF_ERR_V_IS_NEGATIVE */
-        return phi != v_new[0];
+        return si_dne(phi, v_new[0]);
     }
 };
 
@@ -200,34 +194,34 @@ struct ModelSISe3 {
                                                   double t, DC &dc)
     {
         switch (k) {
-        case 0: return gdata[0] * v[0] * si_i2d(u[0]);
-        case 1: return gdata[3] * si_i2d(u[1]);
-        case 2: return gdata[1] * v[0] * si_i2d(u[2]);
-        case 3: return gdata[4] * si_i2d(u[3]);
-        case 4: return gdata[2] * v[0] * si_i2d(u[4]);
-        default: return gdata[5] * si_i2d(u[5]);
+        case 0: return si_mul_i(gdata[0] * v[0], u[0]);
+        case 1: return si_mul_i(gdata[3], u[1]);
+        case 2: return si_mul_i(gdata[1] * v[0], u[2]);
+        case 3: return si_mul_i(gdata[4], u[3]);
+        case 4: return si_mul_i(gdata[2] * v[0], u[4]);
+        default: return si_mul_i(gdata[5], u[5]);
         }
     }
     __device__ __forceinline__ static int pts(double *v_new, const int *u, const double *v,
                                               const double *ldata, const double *gdata,
                                               int node, double t)
     {
-        const int day = (int) t % 365;
-        const double I_n = u[1] + u[3] + u[5];
-        const double n = I_n + u[0] + u[2] + u[4];
+        const int day = si_d2i(t) % 365;
+        const int I_n = u[1] + u[3] + u[5];
+        const long long n = (long long) I_n + u[0] + u[2] + u[4];
         const double phi = v[0];
-        v_new[0] = forward_euler_linear_decay(phi, day, (int) ldata[0], (int) ldata[1],
-                                              (int) ldata[2], (int) ldata[3], gdata[7],
+        v_new[0] = forward_euler_linear_decay(phi, day, si_d2i(ldata[0]), si_d2i(ldata[1]),
+                                              si_d2i(ldata[2]), si_d2i(ldata[3]), gdata[7],
                                               gdata[8], gdata[9], gdata[10]);
-        if (n > 0.0)
-            v_new[0] += gdata[6] * I_n / n + gdata[11];
+        if (n > 0)
+            v_new[0] += si_div(si_mul_i(gdata[6], I_n), si_l2d(n)) + gdata[11];
         else
             v_new[0] += gdata[11];
         if (!isfinite(v_new[0]))
             return -7;
-        if (v_new[0] < 0.0)
+        if (si_bad_rate(v_new[0]))
             return -10;
-        return phi != v_new[0];
+        return si_dne(phi, v_new[0]);
     }
 };
 
@@ -250,7 +244,7 @@ __device__ __forceinline__ double local_spread(const double *neighbors, const do
         for (int k = j * Nc; k < (j + 1) * Nc; k++)
             N_j += u[k];
         if (N_j > 0.0)
-            ls += ((phi[j] * N_j - phi_i_N_i) * D) / (N_i * neighbors[1]);
+            ls += si_div((phi[j] * N_j - phi_i_N_i) * D, N_i * neighbors[1]);
         neighbors += 2;
         j = (int) neighbors[0];
     }
@@ -274,28 +268,28 @@ struct ModelSISe_sp {
                                                   double t, DC &dc)
     {
         if (k == 0)
-            return gdata[0] * v[0] * si_i2d(u[0]);
-        return gdata[1] * si_i2d(u[1]);
+            return si_mul_i(gdata[0] * v[0], u[0]);
+        return si_mul_i(gdata[1], u[1]);
     }
     __device__ __forceinline__ static int pts(double *v_new, const int *u, const double *v,
                                               const double *ldata, const double *gdata,
                                               int node, double t)
     {
-        const int day = (int) t % 365;
-        const double I_i = u[1];
-        const double N_i = u[0] + I_i;
+        const int day = si_d2i(t) % 365;
+        const double I_i = si_i2d(u[1]);
+        const double N_i = si_l2d((long long) u[0] + u[1]);
         const double phi = v[0];
-        v_new[0] = forward_euler_linear_decay(phi, day, (int) ldata[0], (int) ldata[1],
-                                              (int) ldata[2], (int) ldata[3], gdata[3],
+        v_new[0] = forward_euler_linear_decay(phi, day, si_d2i(ldata[0]), si_d2i(ldata[1]),
+                                              si_d2i(ldata[2]), si_d2i(ldata[3]), gdata[3],
                                               gdata[4], gdata[5], gdata[6]);
         if (N_i > 0.0)
-            v_new[0] += gdata[2] * I_i / N_i +
+            v_new[0] += si_div(gdata[2] * I_i, N_i) +
                         local_spread(ldata + 4, v - node, u - 2 * node, N_i, phi, 2, gdata[7]);
         if (!isfinite(v_new[0]))
             return -7;          /* SIMINF_ERR_V_IS_NOT_FINITE */
-        if (v_new[0] < 0.0)
+        if (si_bad_rate(v_new[0]))
             return -10;         /* SIMINF_ERR_V_IS_NEGATIVE */
-        return phi != v_new[0];
+        return si_dne(phi, v_new[0]);
     }
 };
 
@@ -319,21 +313,21 @@ struct ModelSISe3_sp {
                                               const double *ldata, const double *gdata,
                                               int node, double t)
     {
-        const int day = (int) t % 365;
-        const double I_i = u[1] + u[3] + u[5];
-        const double N_i = u[0] + u[2] + u[4] + I_i;
+        const int day = si_d2i(t) % 365;
+        const double I_i = si_i2d(u[1] + u[3] + u[5]);
+        const double N_i = si_i2d(u[0] + u[2] + u[4]) + I_i;
         const double phi = v[0];
-        v_new[0] = forward_euler_linear_decay(phi, day, (int) ldata[0], (int) ldata[1],
-                                              (int) ldata[2], (int) ldata[3], gdata[7],
+        v_new[0] = forward_euler_linear_decay(phi, day, si_d2i(ldata[0]), si_d2i(ldata[1]),
+                                              si_d2i(ldata[2]), si_d2i(ldata[3]), gdata[7],
                                               gdata[8], gdata[9], gdata[10]);
         if (N_i > 0.0)
-            v_new[0] += gdata[6] * I_i / N_i +
+            v_new[0] += si_div(gdata[6] * I_i, N_i) +
                         local_spread(ldata + 4, v - node, u - 6 * node, N_i, phi, 6, gdata[11]);
         if (!isfinite(v_new[0]))
             return -7;
-        if (v_new[0] < 0.0)
+        if (si_bad_rate(v_new[0]))
             return -10;
-        return phi != v_new[0];
+        return si_dne(phi, v_new[0]);
     }
 };
 
@@ -352,9 +346,9 @@ struct ModelSIRmparse {
     {
         if (k == 0) {
             const double N = si_i2d(u[0] + u[1] + u[2]);             /* int sum, as in C */
-            return si_div_cached(gdata[0] * si_i2d(u[0]) * si_i2d(u[1]), N, &dc);
+            return si_div_cached(si_mul_i(si_mul_i(gdata[0], u[0]), u[1]), N, &dc);
         }
-        return gdata[1] * si_i2d(u[1]);
+        return si_mul_i(gdata[1], u[1]);
     }
     __device__ __forceinline__ static int pts(double *, const int *, const double *,
                                               const double *, const double *, int, double)
@@ -378,20 +372,20 @@ struct ModelSISePF {
                                                   double t, DC &dc)
     {
         if (k == 0)
-            return gdata[0] * v[0] * si_i2d(u[0]);
-        return gdata[1] * si_i2d(u[1]);
+            return si_mul_i(gdata[0] * v[0], u[0]);
+        return si_mul_i(gdata[1], u[1]);
     }
     __device__ __forceinline__ static int pts(double *v_new, const int *u, const double *v,
                                               const double *ldata, const double *gdata,
                                               int node, double t)
     {
-        const double S_n = u[0];
-        const double I_n = u[1];
-        const double n = S_n + I_n;
-        v_new[0] = v[0] * (1.0 - 0.03);
-        if (n > 0.0)
-            v_new[0] += 0.05 * I_n / n;
-        return v[0] != v_new[0];
+        const long long n = (long long) u[0] + u[1];
+        const double phi = v[0];
+        double x = phi * (1.0 - 0.03);
+        if (n > 0)
+            x += si_div(si_mul_i(0.05, u[1]), si_l2d(n));
+        v_new[0] = x;
+        return si_dne(phi, x);
     }
 };
 

@@ -35,7 +35,7 @@ enum { MAX_NC = 16, MAX_NT = 32, MAX_ERR = 1024 };
  * the day's longest chains start first, and a thread whose node is done
  * takes the next one.  At most MAX_HEAVY nodes per class and day are
  * listed; the rest come in index order. */
-enum { SSA_BLOCK = 128, HEAVY_CLASSES = 3, MAX_HEAVY = 32768 };
+enum { HORIZON_BLOCK = 128, SSA_BLOCK = 128, HEAVY_CLASSES = 3, MAX_HEAVY = 32768 };
 
 enum { PHASE_INIT = 0, PHASE_SSA = 1, PHASE_E1 = 2, PHASE_E2 = 3, PHASE_PTS = 4 };
 

@@ -611,28 +611,82 @@ SI_HD int si_dge(double a, double b)
     return si_dkey(A) >= si_dkey(B);
 }
 
-/* (double) x for a 32-bit integer, exact, from integer bits. */
+/* (double) x for a 32-bit integer, exact, from integer bits: the leading
+ * one moves to bit 31 and then onto the exponent's lowest bit. */
 SI_HD double si_i2d(int32_t x)
 {
-    if (x == 0)
-        return 0.0;
-    const uint64_t sign = x < 0 ? 0x8000000000000000ULL : 0;
-    const uint64_t m = x < 0 ? (uint64_t) (0u - (uint32_t) x) : (uint64_t) (uint32_t) x;
-    const int p = 63 - si_clz64(m);
-    return si_bits_double(sign | ((uint64_t) (p + 1023) << 52) |
-                          ((m << (52 - p)) & 0x000FFFFFFFFFFFFFULL));
+    const uint32_t m = x < 0 ? 0u - (uint32_t) x : (uint32_t) x;
+    const int c = si_clz32(m) & 31;
+    const uint32_t n = m << c;
+    const uint32_t hi = ((uint32_t) (1022 + 31 - c) << 20) + (n >> 11);
+    const uint64_t b = ((uint64_t) (hi | ((uint32_t) x & 0x80000000u)) << 32) | (n << 21);
+    return si_bits_double(x == 0 ? 0 : b);
 }
 
 /* (double) x for |x| < 2^53, exact, from integer bits. */
 SI_HD double si_l2d(int64_t x)
 {
-    if (x == 0)
-        return 0.0;
+    if (x == (int64_t) (int32_t) x)
+        return si_i2d((int32_t) x);
     const uint64_t sign = x < 0 ? 0x8000000000000000ULL : 0;
     const uint64_t m = x < 0 ? (uint64_t) 0 - (uint64_t) x : (uint64_t) x;
     const int p = 63 - si_clz64(m);
     return si_bits_double(sign | ((uint64_t) (p + 1023) << 52) |
                           ((m << (52 - p)) & 0x000FFFFFFFFFFFFFULL));
+}
+
+/* a * (double) n, correctly rounded, on the integer pipes: the mantissa
+ * times |n| has at most 84 bits, of which the 53 highest are kept and the
+ * rest, at most 32, rounds them (to nearest, ties to even).  A conversion and
+ * a product that hold the FP64 pipe for 64 cycles a warp each become about
+ * 30 integer instructions.  Subnormal, infinite and NaN factors, and
+ * products that may overflow, take the hardware product. */
+SI_HD double si_mul_i(double a, int32_t n)
+{
+    const uint64_t A = si_double_bits(a);
+    const int ea = (int) ((A >> 52) & 0x7FF);
+    const uint64_t sign = (A ^ ((uint64_t) (uint32_t) n << 32)) & 0x8000000000000000ULL;
+    const uint32_t m = n < 0 ? 0u - (uint32_t) n : (uint32_t) n;
+    if (ea == 0 || ea > 2012) {
+        if ((A << 1) == 0)
+            return si_bits_double(sign);
+        return a * si_i2d(n);
+    }
+    const uint32_t alo = (uint32_t) A, ahi = ((uint32_t) (A >> 32) & 0xFFFFFu) | 0x100000u;
+    const uint64_t p0 = (uint64_t) alo * m;
+    const uint64_t p1 = (uint64_t) ahi * m + (p0 >> 32);       /* product / 2^32 */
+    const int s = 43 - si_clz64(p1 | 0x100000u);               /* bits to drop: 0 .. 32 */
+    const uint64_t low = (uint64_t) (uint32_t) p0 << (32 - s);
+    uint64_t mant = (p1 << (32 - s)) | (low >> 32);
+    const uint32_t frac = (uint32_t) low;
+    mant += (frac > 0x80000000u) | ((frac == 0x80000000u) & (uint32_t) mant & 1u);
+    const uint64_t b = ((uint64_t) (ea + s - 1) << 52) + mant;  /* a carry moves up */
+    return si_bits_double(sign | (m == 0 ? 0 : b));
+}
+
+/* (int) x, from the bits where |x| < 2^31. */
+SI_HD int si_d2i(double x)
+{
+    const uint64_t b = si_double_bits(x);
+    const int e = (int) ((b >> 52) & 0x7FF) - 1023;
+    if (e > 30)
+        return (int) x;
+    const uint64_t m = (b & 0x000FFFFFFFFFFFFFULL) | 0x0010000000000000ULL;
+    const int v = e < 0 ? 0 : (int) (m >> (52 - e));
+    return b >> 63 ? -v : v;
+}
+
+/* a != b with IEEE semantics (true when either is NaN). */
+SI_HD int si_dne(double a, double b)
+{
+    const uint64_t A = si_double_bits(a), B = si_double_bits(b);
+    return si_isnan_bits(A) || (A != B && ((A | B) << 1) != 0);
+}
+
+/* a >= b for doubles neither of which is NaN. */
+SI_HD int si_dge_num(double a, double b)
+{
+    return si_dkey(si_double_bits(a)) >= si_dkey(si_double_bits(b));
 }
 
 /* !isfinite(x) || x < 0.0, the reference's invalid-rate test. */
@@ -771,7 +825,14 @@ SI_HD double si_div_r(double a, const si_recip *r, double b)
 {
     int special = 0;
     const double q = si_div_r_spec(a, r, &special);
-    return special ? a / b : q;
+    if (special) {
+        /* a zero numerator (no one to infect, no one infected) is common */
+        const uint64_t A = si_double_bits(a);
+        if ((A << 1) == 0 && r->mb != 0)
+            return si_bits_double((A ^ r->B) & 0x8000000000000000ULL);
+        return a / b;
+    }
+    return q;
 }
 
 SI_HD double si_div(double a, double b)
