@@ -1581,6 +1581,7 @@ static cudaError_t launch_all(siminf_gpu_plan *p, DevState s, cudaStream_t st, K
     if (p->horizon)
         return timed(kp, 4, st, [&] { return L->horizon(s, p->d_days, ndays, st); });
     e = timed(kp, 0, st, [&] { return e1_start(s, st); });
+    s.chained = kp == nullptr;          /* one day's kernels behind another, nothing between */
     for (int d = 0; d < ndays && e == cudaSuccess; d++) {
         const DayInfo &di = p->days[d];
         if (s.two_pass && !s.aem)
@@ -1943,11 +1944,15 @@ static cudaError_t launch_streamed(siminf_gpu_plan *p, DevState s, cudaStream_t 
             e = e1_start(s, st);        /* the run's E1 list, or the chunk's */
         for (int d = d0; d < d1 && e == cudaSuccess; d++) {
             const DayInfo &di = p->days[d];
-            if (s.two_pass && !s.aem)
+            s.chained = d > d0;         /* not behind the chunk's copies */
+            if (s.two_pass && !s.aem) {
                 e = L->quick(s, d, di.tt, di.next, st);
+                s.chained = 1;
+            }
             if (e == cudaSuccess)
                 e = s.aem ? L->aem_day(s, d, di.tt, di.next, st)
                           : L->ssa_e1(s, d, di.tt, di.next, st);
+            s.chained = 1;
             if (e == cudaSuccess) {
                 const std::vector<long long> &cnt = p->day_waves[d];
                 std::vector<long long> off(cnt.size());
@@ -2365,11 +2370,15 @@ static cudaError_t launch_streamed_dev(siminf_gpu_plan *p, DevState s, cudaStrea
             p->e2_day_off[d] = pl.base2 + pl.ch.off[j];
             p->e2_day_off[d + 1] = pl.base2 + pl.ch.off[j + 1];
             p->day_waves[d] = pl.ch.waves[j];
-            if (s.two_pass && !s.aem)
+            s.chained = d > d0;         /* not behind the chunk's copies */
+            if (s.two_pass && !s.aem) {
                 e = L->quick(s, d, di.tt, di.next, st);
+                s.chained = 1;
+            }
             if (e == cudaSuccess)
                 e = s.aem ? L->aem_day(s, d, di.tt, di.next, st)
                           : L->ssa_e1(s, d, di.tt, di.next, st);
+            s.chained = 1;
             if (e == cudaSuccess) {
                 const std::vector<long long> &cnt = p->day_waves[d];
                 std::vector<long long> off(cnt.size());

@@ -173,6 +173,10 @@ struct DevState {
      * nodes are not stepped by groups of lanes. */
     int heavy_lanes;
 
+    /* The launch may start while the kernel before it drains (host only;
+     * off for the first kernel behind another stream's event). */
+    int chained;
+
     /* Profiling: per day, the most transitions any node fired that day
      * (nullptr: not recorded). */
     unsigned *day_max;
