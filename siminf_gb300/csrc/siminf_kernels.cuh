@@ -2118,21 +2118,18 @@ __device__ __forceinline__ void e2_apply(const DevState &s, const E2Rec &e, int 
              * 139-160); the urn of each compartment is si_hypergeometric's */
             unsigned at = (unsigned) r.ctr & 3u;        /* the next draw's word */
             int left = total, want = n;
-            for (unsigned rows = cols;; rows &= rows - 1) {
-                const int row = __ffs((int) rows) - 1;
-                int nk = uu[0];
 #pragma unroll
-                for (int c = 1; c < NC; c++)
-                    if (c == row)
-                        nk = uu[c];
-                const bool last = want == 0 || (rows & (rows - 1)) == 0;
-                int k = want;
-                if (!last) {
-                    const bool complement = 2 * (long long) want > left;
+            for (int c = 0; c < NC; c++) {
+                if (!((cols >> c) & 1u))
+                    continue;
+                const int nk = uu[c];
+                if (cols >> c == 1u) {
+                    ind[c] = want;                      /* the last compartment */
+                } else if (nk > 0 && want > 0) {
+                    const bool complement = (unsigned) want > (unsigned) (left - want);
                     const int t = complement ? left - want : want;
                     unsigned a = (unsigned) nk, rem = (unsigned) left;
-                    int i = 0;
-                    k = 0;
+                    int i = 0, k = 0;
                     while (i < t && a > 0 && a < rem) {
                         if (at == E2_WORDS) {
                             blk += E2_WORDS / 4;
@@ -2151,15 +2148,10 @@ __device__ __forceinline__ void e2_apply(const DevState &s, const E2Rec &e, int 
                     if (a > 0 && a == rem)
                         k += t - i;
                     k = complement ? nk - k : k;
+                    ind[c] = k;
+                    want -= k;
                 }
-#pragma unroll
-                for (int c = 0; c < NC; c++)
-                    if (c == row)
-                        ind[c] = k;
-                if (last)
-                    break;
                 left -= nk;
-                want -= k;
             }
             s.ctr[gs] = (blk << 2) + at;
         }
