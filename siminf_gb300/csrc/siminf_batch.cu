@@ -25,6 +25,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <thread>
 #include <vector>
 
@@ -213,68 +214,115 @@ extern "C" int siminf_gpu_run_batch(siminf_gpu_batch_job *jobs, int njobs,
     }
 
     /* Events: stable counting sort by (time, E2 after E1), each model's own
-     * order kept, events past a model's horizon dropped.  Keys are counted
-     * per model on host threads, offsets run key-major then model-major,
-     * and every model then writes its own events. */
-    const int nthreads = std::max(1, std::min(njobs, (int) std::thread::hardware_concurrency()));
-    std::vector<int> jmin(njobs, INT_MAX), jmax(njobs, INT_MIN), jbad(njobs, 0);
-    std::vector<long long> jcount(njobs, 0);
-    auto for_jobs = [&](auto &&f) {
+     * order kept, events past a model's horizon dropped.  Offsets run
+     * key-major then model-major.  The events of the largest models are most
+     * of the table, so host threads work on slices of SLICE events: they
+     * check a slice and note where its key changes, and then write it, each
+     * run of one key from that run's offset on.  A model whose events are
+     * not in order is counted and written event by event, by one thread.
+     * The merged columns start uninitialised: the threads that write them
+     * touch their pages first. */
+    enum { SLICE = 1 << 17 };
+    struct Slice {
+        int j, lo, hi, bad = 0, tmin = INT_MAX, tmax = INT_MIN;
+        bool ordered = true;
+        long long count = 0;
+        std::vector<int> starts;        /* events whose key differs from the one before */
+    };
+    std::vector<Slice> slices;
+    for (int j = 0; j < njobs; j++)
+        for (long long lo = 0; lo < jobs[j].args->len; lo += SLICE) {
+            slices.emplace_back();
+            slices.back().j = j;
+            slices.back().lo = (int) lo;
+            slices.back().hi = (int) std::min(lo + SLICE, (long long) jobs[j].args->len);
+        }
+    const int nthreads =
+        std::max(1, std::min((int) slices.size(), (int) std::thread::hardware_concurrency()));
+    auto on_threads = [&](int n, auto &&f) {
         std::atomic<int> next(0);
+        auto work = [&]() {
+            for (int k = next++; k < n; k = next++)
+                f(k);
+        };
         std::vector<std::thread> th;
-        for (int t = 0; t < nthreads; t++)
-            th.emplace_back([&]() {
-                for (int j = next++; j < njobs; j = next++)
-                    f(j);
-            });
+        for (int t = 1; t < nthreads; t++)
+            th.emplace_back(work);
+        work();
         for (auto &x : th)
             x.join();
     };
-    for_jobs([&](int j) {
-        const siminf_gpu_solver_args *a = jobs[j].args;
-        for (int i = 0; i < a->len; i++) {
-            if (event_day(a->time[i]) >= ndays[j])
+    auto is_e2 = [](const siminf_gpu_solver_args *a, int i) {
+        return a->event[i] == SIMINF_GPU_EXTERNAL_TRANSFER_EVENT;
+    };
+    on_threads((int) slices.size(), [&](int k) {
+        Slice &s = slices[k];
+        const siminf_gpu_solver_args *a = jobs[s.j].args;
+        for (int i = s.lo; i < s.hi; i++) {
+            const bool e2 = is_e2(a, i);
+            if (i == 0) {
+                s.starts.push_back(i);
+            } else if (a->time[i] != a->time[i - 1] || e2 != is_e2(a, i - 1)) {
+                s.starts.push_back(i);
+                s.ordered &= a->time[i] > a->time[i - 1] || (a->time[i] == a->time[i - 1] && e2);
+            }
+            if (event_day(a->time[i]) >= ndays[s.j])
                 continue;
-            const bool e2 = a->event[i] == SIMINF_GPU_EXTERNAL_TRANSFER_EVENT;
             if (a->node[i] < 1 || a->node[i] > a->Nn ||
                 (e2 && (a->dest[i] < 1 || a->dest[i] > a->Nn))) {
-                if (!jbad[j])
-                    jbad[j] = (e2 && a->node[i] >= 1 && a->node[i] <= a->Nn) ? -(i + 1) : i + 1;
+                if (!s.bad)
+                    s.bad = (e2 && a->node[i] >= 1 && a->node[i] <= a->Nn) ? -(i + 1) : i + 1;
                 continue;
             }
-            jmin[j] = std::min(jmin[j], a->time[i]);
-            jmax[j] = std::max(jmax[j], a->time[i]);
-            jcount[j]++;
+            s.tmin = std::min(s.tmin, a->time[i]);
+            s.tmax = std::max(s.tmax, a->time[i]);
+            s.count++;
         }
     });
     long long nev = 0;
     int tmin = INT_MAX, tmax = INT_MIN;
-    for (int j = 0; j < njobs; j++) {
-        if (jbad[j]) {
-            snprintf(msg, sizeof(msg), "batch job %d: event %d names a node outside it", j,
-                     std::abs(jbad[j]));
-            return fail(jbad[j] < 0 ? SIMINF_GPU_ERR_DEST_OUT_OF_BOUNDS
-                                    : SIMINF_GPU_ERR_NODE_OUT_OF_BOUNDS, msg);
+    std::vector<char> ordered(njobs, 1);
+    for (const Slice &s : slices) {
+        if (s.bad) {
+            snprintf(msg, sizeof(msg), "batch job %d: event %d names a node outside it", s.j,
+                     std::abs(s.bad));
+            return fail(s.bad < 0 ? SIMINF_GPU_ERR_DEST_OUT_OF_BOUNDS
+                                  : SIMINF_GPU_ERR_NODE_OUT_OF_BOUNDS, msg);
         }
-        nev += jcount[j];
-        tmin = std::min(tmin, jmin[j]);
-        tmax = std::max(tmax, jmax[j]);
+        nev += s.count;
+        tmin = std::min(tmin, s.tmin);
+        tmax = std::max(tmax, s.tmax);
+        ordered[s.j] &= s.ordered;
     }
-    std::vector<int> ev_event(nev), ev_time(nev), ev_node(nev), ev_dest(nev), ev_n(nev),
-        ev_select(nev), ev_shift(nev);
-    std::vector<double> ev_prop(nev);
+    const size_t nalloc = (size_t) std::max(nev, 1LL);
+    std::unique_ptr<int[]> ev_event(new int[nalloc]), ev_time(new int[nalloc]),
+        ev_node(new int[nalloc]), ev_dest(new int[nalloc]), ev_n(new int[nalloc]),
+        ev_select(new int[nalloc]), ev_shift(new int[nalloc]);
+    std::unique_ptr<double[]> ev_prop(new double[nalloc]);
     if (nev > 0) {
         const long long nkeys = 2 * ((long long) tmax - tmin + 1);
         if (nkeys * njobs > 400000000LL)
             return fail(SIMINF_GPU_ERR_INVALID_MODEL, "batch event times span too wide a range");
         auto key = [&](const siminf_gpu_solver_args *a, int i) {
-            return 2 * ((long long) a->time[i] - tmin) +
-                   (a->event[i] == SIMINF_GPU_EXTERNAL_TRANSFER_EVENT ? 1 : 0);
+            return 2 * ((long long) a->time[i] - tmin) + (is_e2(a, i) ? 1 : 0);
         };
         /* off[key * njobs + j]: first position of model j's events with key */
         std::vector<long long> off((size_t) nkeys * njobs, 0);
-        for_jobs([&](int j) {
+        std::vector<std::vector<int>> starts(njobs);
+        for (const Slice &s : slices)
+            if (ordered[s.j])
+                starts[s.j].insert(starts[s.j].end(), s.starts.begin(), s.starts.end());
+        on_threads(njobs, [&](int j) {
             const siminf_gpu_solver_args *a = jobs[j].args;
+            if (ordered[j]) {
+                for (size_t k = 0; k < starts[j].size(); k++) {
+                    const int i = starts[j][k];
+                    const int end = k + 1 < starts[j].size() ? starts[j][k + 1] : a->len;
+                    if (event_day(a->time[i]) < ndays[j])
+                        off[(size_t) key(a, i) * njobs + j] = end - i;
+                }
+                return;
+            }
             for (int i = 0; i < a->len; i++)
                 if (event_day(a->time[i]) < ndays[j])
                     off[(size_t) key(a, i) * njobs + j]++;
@@ -285,22 +333,37 @@ extern "C" int siminf_gpu_run_batch(siminf_gpu_batch_job *jobs, int njobs,
             off[k] = run;
             run += c;
         }
-        for_jobs([&](int j) {
-            const siminf_gpu_solver_args *a = jobs[j].args;
-            const int base = (int) node0[j];
-            for (int i = 0; i < a->len; i++) {
-                if (event_day(a->time[i]) >= ndays[j])
-                    continue;
-                const long long at = off[(size_t) key(a, i) * njobs + j]++;
-                const bool e2 = a->event[i] == SIMINF_GPU_EXTERNAL_TRANSFER_EVENT;
-                ev_event[at] = a->event[i];
-                ev_time[at] = a->time[i];
-                ev_node[at] = a->node[i] + base;
-                ev_dest[at] = e2 ? a->dest[i] + base : a->dest[i];
-                ev_n[at] = a->n[i];
-                ev_prop[at] = a->proportion[i];
-                ev_select[at] = a->select[i];
-                ev_shift[at] = a->shift[i];
+        auto write = [&](const siminf_gpu_solver_args *a, int base, int i, long long at) {
+            const bool e2 = is_e2(a, i);
+            ev_event[at] = a->event[i];
+            ev_time[at] = a->time[i];
+            ev_node[at] = a->node[i] + base;
+            ev_dest[at] = e2 ? a->dest[i] + base : a->dest[i];
+            ev_n[at] = a->n[i];
+            ev_prop[at] = a->proportion[i];
+            ev_select[at] = a->select[i];
+            ev_shift[at] = a->shift[i];
+        };
+        on_threads((int) slices.size(), [&](int k) {
+            const Slice &s = slices[k];
+            const siminf_gpu_solver_args *a = jobs[s.j].args;
+            const int base = (int) node0[s.j];
+            if (!ordered[s.j]) {
+                /* the model's first slice writes all of it, in its order */
+                for (int i = 0; s.lo == 0 && i < a->len; i++)
+                    if (event_day(a->time[i]) < ndays[s.j])
+                        write(a, base, i, off[(size_t) key(a, i) * njobs + s.j]++);
+                return;
+            }
+            const std::vector<int> &st = starts[s.j];
+            size_t r = (size_t) (std::upper_bound(st.begin(), st.end(), s.lo) - st.begin()) - 1;
+            for (int i = s.lo; i < s.hi; r++) {
+                const int end = std::min(s.hi, r + 1 < st.size() ? st[r + 1] : a->len);
+                if (event_day(a->time[i]) >= ndays[s.j])
+                    return;                     /* times ascend: so does the rest */
+                const long long at = off[(size_t) key(a, i) * njobs + s.j] - st[r];
+                for (; i < end; i++)
+                    write(a, base, i, at + i);
             }
         });
     }
@@ -317,14 +380,14 @@ extern "C" int siminf_gpu_run_batch(siminf_gpu_batch_job *jobs, int njobs,
     m.irU = m.jcU = m.irV = m.jcV = nullptr;
     m.prU = m.prV = nullptr;
     m.len = (int) nev;
-    m.event = ev_event.data();
-    m.time = ev_time.data();
-    m.node = ev_node.data();
-    m.dest = ev_dest.data();
-    m.n = ev_n.data();
-    m.proportion = ev_prop.data();
-    m.select = ev_select.data();
-    m.shift = ev_shift.data();
+    m.event = ev_event.get();
+    m.time = ev_time.get();
+    m.node = ev_node.get();
+    m.dest = ev_dest.get();
+    m.n = ev_n.get();
+    m.proportion = ev_prop.get();
+    m.select = ev_select.get();
+    m.shift = ev_shift.get();
     if (eref >= 0) {
         m.irE = jobs[eref].args->irE;
         m.jcE = jobs[eref].args->jcE;

@@ -41,7 +41,15 @@
 #include <tuple>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <cuda_runtime.h>
+
+/* Linux 5.14; older C libraries' headers do not name it */
+#ifndef MADV_POPULATE_WRITE
+#define MADV_POPULATE_WRITE 23
+#endif
 #include <dlfcn.h>
 
 #include "../../include/siminf_gb300.h"
@@ -447,11 +455,19 @@ static int planner_threads()
     return (int) n;
 }
 
-/* Run f(t, n) on n = planner_threads() threads and join. */
-template <class F>
-static void parallel(F &&f)
+/* Threads for so many items: one for each 16,384, at most
+ * planner_threads().  Starting fifteen threads takes 0.6 ms, more than the
+ * whole of a plan without events. */
+static int threads_for(long long items)
 {
-    const unsigned n = (unsigned) planner_threads();
+    return (int) std::min((long long) planner_threads(), items / 16384 + 1);
+}
+
+/* Run f(t, n) on n = threads_for(items) threads and join. */
+template <class F>
+static void parallel(long long items, F &&f)
+{
+    const unsigned n = (unsigned) threads_for(items);
     std::vector<std::thread> th;
     for (unsigned t = 1; t < n; t++)
         th.emplace_back([&f, t, n] { f((int) t, (int) n); });
@@ -480,9 +496,9 @@ static int plan_scan(siminf_gpu_plan *p, const siminf_gpu_solver_args *a, int ns
         std::vector<long long> e2_per_day;
         std::vector<PlannedErr> planned;
     };
-    std::vector<Chunk> chunks(planner_threads());
+    std::vector<Chunk> chunks(threads_for(len));
     const int E2 = SIMINF_GPU_EXTERNAL_TRANSFER_EVENT;
-    parallel([&](int t, int n) {
+    parallel(len, [&](int t, int n) {
         Chunk &c = chunks[t];
         c.e2_per_day.assign(ndays + 1, 0);
         const long long lo = len * t / n, hi = len * (t + 1) / n;
@@ -943,7 +959,7 @@ static int plan_events(siminf_gpu_plan *p, const siminf_gpu_solver_args *a, int 
     e2.reset(new E2Rec[p->e2_count > 0 ? p->e2_count : 1]);
     std::atomic<int> next_day(0);
     E2Rec *dst = e2.get();
-    parallel([&](int, int) {
+    parallel((long long) p->e2_count, [&](int, int) {
         WaveTracker w(a->Nn);
         for (int d = next_day++; d < p->ndays; d = next_day++)
             plan_day_waves(p, a, d, w, dst, p->e2_day_off[d]);
@@ -2560,6 +2576,54 @@ static bool build_run_graph(siminf_gpu_plan *p, const DevState &s)
     return true;
 }
 
+/* Pages of a call's host output arrays, made present beside the GPU's work:
+ * arrays fresh from the allocator have none, and the copy back would fault
+ * them in one by one (288 MB: 54 ms, against 10 ms for the copy alone; 65 MB:
+ * 27 ms, against 0.2).  Contents stay as they are; a kernel without
+ * MADV_POPULATE_WRITE leaves everything to the copy.  Started once the run's
+ * launches are queued: before, its hold on the memory map slows the threads
+ * that plan and launch (100,000 nodes x 180 days: 22.7 ms of solve, then
+ * 30.5). */
+struct siminf::PresentPages {
+private:
+    std::vector<std::pair<char *, size_t>> parts;
+    std::vector<std::thread> threads;
+    std::atomic<size_t> next{0};
+
+public:
+    ~PresentPages() { join(); }
+    void add(const void *p, size_t bytes)
+    {
+        enum { PART = 4 << 20, LEAST = 8 << 20 };
+        if (!p || bytes < LEAST || host_pinned(p))
+            return;
+        const size_t page = (size_t) sysconf(_SC_PAGESIZE);
+        const uintptr_t lo = ((uintptr_t) p + page - 1) / page * page,
+                        hi = ((uintptr_t) p + bytes) / page * page;
+        for (uintptr_t q = lo; q < hi; q += PART)
+            parts.emplace_back((char *) q, (size_t) std::min((uintptr_t) PART, hi - q));
+    }
+    void start()
+    {
+        const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+        /* two threads: eight take three times as long, on the process's
+         * memory map */
+        const size_t n = std::min((size_t) 2, parts.size());
+        for (size_t t = 0; t < n; t++)
+            threads.emplace_back([this] {
+                for (size_t k = next++; k < parts.size(); k = next++)
+                    if (madvise(parts[k].first, parts[k].second, MADV_POPULATE_WRITE))
+                        return;
+            });
+    }
+    void join()
+    {
+        for (auto &t : threads)
+            t.join();
+        threads.clear();
+    }
+};
+
 extern "C" {
 
 static int plan_run_impl(siminf_gpu_plan *p, cudaStream_t st, KernelProfile *kp)
@@ -2628,6 +2692,8 @@ static int plan_run_impl(siminf_gpu_plan *p, cudaStream_t st, KernelProfile *kp)
     }
     if (e != cudaSuccess)
         return cuda_fail(e, "kernel launch");
+    if (p->pages)
+        p->pages->start();
     e = cudaEventRecord(ev.b, st);
     if (e == cudaSuccess)
         e = cudaEventSynchronize(ev.b);
@@ -3498,16 +3564,23 @@ static int run_solver(siminf_gpu_solver_args *args, const siminf_gpu_model *mode
                       const siminf_gpu_options *opt)
 {
     siminf_gpu_plan *p = nullptr;
+    PresentPages pages;
     /* streamed: the external transfers' waves are planned and copied
      * while the GPU runs the earlier days */
     int rc = plan_create_impl(args, model, opt, &p, true);
     if (rc)
         return rc;
+    pages.add(args->U ? (const void *) args->U : args->prU,
+              args->U ? p->U_len * sizeof(int) : p->prU_len * sizeof(double));
+    pages.add(args->V ? (const void *) args->V : args->prV,
+              args->V ? p->V_len * sizeof(double) : p->prV_len * sizeof(double));
+    p->pages = &pages;
     /* pinned outputs come back chunk by chunk during the run */
     if (p->e2_pending && host_pinned(args->U ? (const void *) args->U : args->prU) &&
         (p->s.Nd == 0 || host_pinned(args->V ? (const void *) args->V : args->prV)))
         p->out_args = args;
     rc = plan_run_impl(p, p->stream, nullptr);
+    pages.join();
     if (!rc && p->out_args) {
         auto t0 = std::chrono::steady_clock::now();
         cudaError_t e = download_columns(p, args, p->cols_sent, p->s.tlen, p->stream);

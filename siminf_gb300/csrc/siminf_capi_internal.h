@@ -32,6 +32,10 @@ struct PlannedErr {
     int day, code, index, node, phase;
 };
 
+namespace siminf {
+struct PresentPages;        /* siminf_capi.cpp */
+}
+
 struct siminf_gpu_plan {
     const Launchers *L = nullptr;
     DevState s{};
@@ -54,6 +58,7 @@ struct siminf_gpu_plan {
 
     /* host-side copies needed to write results back */
     size_t U_len = 0, V_len = 0, prU_len = 0, prV_len = 0;
+    siminf::PresentPages *pages = nullptr;  /* host outputs to make present during the run */
     int *d_u0 = nullptr;            /* device copy of the initial state */
     double *d_v0 = nullptr;
     double tt0 = 0;
