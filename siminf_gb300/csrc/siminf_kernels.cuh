@@ -2391,11 +2391,11 @@ __global__ void __launch_bounds__(256) k_pts_store(DevState s, int day, double t
 #define AEM_SID (1ULL << 63)
 
 __device__ __forceinline__ double aem_neglog(uint64_t seed, long long g, int Nt, int j,
-                                             uint64_t &ctr)
+                                             uint64_t &ctr, const si_nl_tables *nl)
 {
     si_rng r;
     si_rng_init(&r, seed, AEM_SID | ((uint64_t) g * (uint64_t) Nt + (uint64_t) j), ctr);
-    const double x = si_neglog_u32(si_next_u32(&r));
+    const double x = si_neglog_u32_in(si_next_u32(&r), nl);
     ctr = r.ctr;
     return x;
 }
@@ -2407,7 +2407,8 @@ __device__ __forceinline__ double aem_neglog(uint64_t seed, long long g, int Nt,
  * exactly, so tt + q and q + tt are the same double. */
 __device__ __forceinline__ void aem_calc_times(double &time, double &inf, double tt,
                                                double old_rate, double new_rate, uint64_t seed,
-                                               long long g, int Nt, int j, uint64_t &ctr)
+                                               long long g, int Nt, int j, uint64_t &ctr,
+                                               const si_nl_tables *nl)
 {
     const double oldtime = time;
     int kind;                           /* 0: q + tt, 1: q * (oldtime - tt) + tt, 2: none */
@@ -2439,7 +2440,7 @@ __device__ __forceinline__ void aem_calc_times(double &time, double &inf, double
     if (kind == 2)
         return;
     if (draw)
-        num = aem_neglog(seed, g, Nt, j, ctr);
+        num = aem_neglog(seed, g, Nt, j, ctr, nl);
     const double q = si_div(num, new_rate);
     time = kind == 0 ? q + tt : (q * (oldtime - tt)) + tt;
 }
@@ -2479,7 +2480,7 @@ __device__ __forceinline__ int aem_init_node(const DevState &s, long long g, dou
         if (!isfinite(rate) || rate < 0.0)
             record_error(s, ERR_INVALID_RATE, PHASE_INIT, 0, g, j, -1, tt0, rate);
         uint64_t c = 0;
-        double t = si_div(aem_neglog(s.seed, g, NT, j, c), rate) + tt0;
+        double t = si_div(aem_neglog(s.seed, g, NT, j, c, SI_NL_GLOBAL), rate) + tt0;
         if (t <= 0.0)
             t = si_bits_double(0x7FF0000000000000ULL);
         s.react_time[k] = t;
@@ -2493,7 +2494,7 @@ __device__ __forceinline__ int aem_init_node(const DevState &s, long long g, dou
     return heavy_class<M>(s, sum);
 }
 
-/* The state of one node's aem day, held by one thread. */
+/* One node's state in k_aem_pts. */
 template <class M>
 struct AemNode {
     int u[M::NC];
@@ -2519,125 +2520,47 @@ __device__ __forceinline__ void aem_refresh(const DevState &s, AemNode<M> &a, lo
         a.err_t = t;
         a.err_rate = nr;
     }
-    aem_calc_times(a.time[j], a.inf[j], tc, old, nr, s.seed, g, M::NT, j, a.ctr[j]);
+    aem_calc_times(a.time[j], a.inf[j], tc, old, nr, s.seed, g, M::NT, j, a.ctr[j],
+                   SI_NL_GLOBAL);
 }
 
-/* One aem step of a node at its day (src/solvers/SimInf_solver_aem.c:
- * 179-307): the transition with the smallest event time fires, then its
- * dependents in G's column (row order) and itself get new rates and event
- * times.  Returns true when the next event falls past the day's end. */
+/* Lanes a node has in k_aem_day: one a transition, to a power of two. */
 template <class M>
-__device__ __forceinline__ bool aem_step(const DevState &s, AemNode<M> &a, long long g,
-                                         double next, const double *v, const double *ld,
-                                         const double *gd, const int *sS, const uint32_t *sG,
-                                         unsigned &fired, si_recip &dc)
-{
-    constexpr int NC = M::NC, NT = M::NT;
-    int tr = 0;
-    double t = a.time[0];
-#pragma unroll
-    for (int j = 1; j < NT; j++)
-        if (a.time[j] < t) {
-            t = a.time[j];
-            tr = j;
-        }
-    if (isinf(t) || t >= next)
-        return true;
-    if (++fired > s.max_fired) {
-        a.err = ERR_TIMEOUT;
-        a.err_tr = tr;
-        a.err_t = t;
-        return true;
-    }
-    int neg = 0;
-#pragma unroll
-    for (int c = 0; c < NC; c++) {
-        const int d = sS[tr * NC + c];
-        a.u[c] += d;
-        neg |= (d != 0) & (a.u[c] < 0);
-    }
-    if (neg) {
-        a.err = ERR_NEGATIVE_STATE;
-        a.err_tr = tr;
-        a.err_t = t;
-        a.err_rate = 0.0;
-    }
-    const uint32_t gm = sG[tr];
-#pragma unroll
-    for (int j = 0; j < NT; j++)
-        if (j != tr && (gm & (1u << j)))
-            aem_refresh<M>(s, a, g, j, v, ld, gd, t, t, dc);
-#pragma unroll
-    for (int j = 0; j < NT; j++)
-        if (j == tr)
-            aem_refresh<M>(s, a, g, j, v, ld, gd, t, t, dc);
-    return false;
-}
+struct AemLanes {
+    static constexpr int value = M::NT <= 1    ? 1
+                                 : M::NT <= 2  ? 2
+                                 : M::NT <= 4  ? 4
+                                 : M::NT <= 8  ? 8
+                                 : M::NT <= 16 ? 16
+                                               : 32;
+};
 
-/* The end of a node's aem day: its error, or its E1 events; the state
- * written back with t = next. */
+/* One day of every node under the all-events method, then its E1 events: a
+ * persistent grid whose groups of AemLanes lanes take nodes from the
+ * day's work queue, first the heavy nodes (rate sum >= heavy_rate at the
+ * start of the day, listed by the previous day's end, heaviest class first),
+ * then every other node in index order.  Lane j of a group holds transition
+ * j's rate, event time, sleeping time and stream (src/solvers/
+ * SimInf_solver_aem.c:179-307): the group finds the smallest event time (the
+ * lowest transition among equal ones), every lane applies that transition
+ * to its copy of u, and the transition and its dependents in G's column
+ * each refresh their own rate and time, side by side: one division a step
+ * where one lane did NT of them one after the other.  Bound: the busiest
+ * node's chain.  SEIR, 100,000 nodes x 120 days: 50.3 ms with a lane a node,
+ * 26.3 with four. */
 template <class M>
-__device__ __forceinline__ void aem_finish(const DevState &s, AemNode<M> &a, long long g, int day,
-                                           double tt, double next)
+__global__ void __launch_bounds__(SSA_BLOCK, 4) k_aem_day(DevState s, int day, double tt,
+                                                          double next)
 {
-    constexpr int NC = M::NC, NT = M::NT;
-    si_rng r;
-    {
-        uint64_t seed, sid;
-        stream_key(s, g, seed, sid);
-        si_rng_init(&r, seed, sid, s.ctr[g]);
-    }
-    if (a.err) {
-        record_error(s, a.err, PHASE_SSA, day, g, a.err_tr, -1, a.err_t, a.err_rate);
-    } else {
-        int e_code = 0, e_idx = -1;
-        int2 at = s.e1_next[g];
-        if (node_e1<NC>(s, a.u, at, node_of(s, g), day, r, e_code, e_idx)) {
-            s.update[g] = 1;
-            s.e1_next[g] = at;
-        }
-        if (e_code)
-            record_error(s, e_code, PHASE_E1, day, g, -1, e_idx, tt, 0);
-    }
-    store_u<NC>(s.u + g * NC, a.u);
-#pragma unroll
-    for (int j = 0; j < NT; j++) {
-        const size_t k = (size_t) j * s.Ntot + g;
-        s.t_rate[k] = a.rate[j];
-        s.react_time[k] = a.time[j];
-        s.react_inf[k] = a.inf[j];
-        s.react_ctr[k] = a.ctr[j];
-    }
-    s.t_time[g] = next;
-    s.ctr[g] = r.ctr;
-}
-
-/* One day of every node under the all-events method, then its E1 events:
- * a persistent grid fed by the day's work queue, as k_ssa_e1 -- first the
- * heavy nodes (rate sum >= heavy_rate at the start of the day, listed by
- * the previous day's end, heaviest class first), 32 to a warp that runs
- * them to the day's end in a tight loop, then every other node in index
- * order, lane by lane, a lane whose node's day is over taking the next
- * node at once.  One atomic per warp hands out the entries. */
-template <class M>
-__global__ void __launch_bounds__(SSA_BLOCK, M::NT <= 4 ? 4 : 3) k_aem_day(DevState s, int day,
-                                                                          double tt, double next)
-{
-    constexpr int NC = M::NC, NT = M::NT, ND = M::ND;
+    constexpr int NC = M::NC, NT = M::NT, ND = M::ND, G = AemLanes<M>::value;
     __shared__ int sS[NT * NC];
     __shared__ uint32_t sG[NT];
+    __shared__ __align__(16) si_nl_tables nl;
+    load_nl_smem(nl);
     load_model_smem<M>(s, sS, sG);
     day_begin();
     const int par = day & 1, npar = (day + 1) & 1;
-    if (blockIdx.x == 0 && threadIdx.x < HEAVY_CLASSES)
-        s.heavy_count[npar * HEAVY_CLASSES + threadIdx.x] = 0;  /* filled by this day's end */
-    if (blockIdx.x == 0 && threadIdx.x < 2)
-        s.queue_next[npar * 2 + threadIdx.x] = 0;
-    unsigned long long fired = 0;
-    if (load_flag(s.err_day) < day) {
-        add_fired(s, fired);
-        return;
-    }
+    const int err_day = load_flag(s.err_day);
     int n[HEAVY_CLASSES];
     unsigned long long H = 0;
 #pragma unroll
@@ -2645,91 +2568,178 @@ __global__ void __launch_bounds__(SSA_BLOCK, M::NT <= 4 ? 4 : 3) k_aem_day(DevSt
         n[c] = min(s.heavy_count[par * HEAVY_CLASSES + c], (int) MAX_HEAVY);
         H += (unsigned long long) n[c];
     }
-    const unsigned long long Ntot = (unsigned long long) s.Ntot;
-    const int lane = threadIdx.x & 31;
+    if (blockIdx.x == 0 && threadIdx.x < HEAVY_CLASSES)
+        s.heavy_count[npar * HEAVY_CLASSES + threadIdx.x] = 0;  /* filled by this day's end */
+    if (blockIdx.x == 0 && threadIdx.x < 2)
+        s.queue_next[npar * 2 + threadIdx.x] = 0;
+    unsigned long long fired = 0;
+    if (err_day < day) {
+        add_fired(s, fired);
+        return;
+    }
     const unsigned FULL = 0xFFFFFFFFu;
-    AemNode<M> a;
-    long long g = -1;
-    bool alive = true, need = true, heavy = false;
-    bool heavy_left = H > 0;            /* warp-uniform: the heavy part may have entries */
+    const int lane = threadIdx.x & 31, j = lane & (G - 1), base = lane - j;
+    const unsigned group = (G == 32 ? FULL : ((1u << (G & 31)) - 1u)) << base;
+    const bool own = j < NT;                /* the lane holds a transition */
+    long long g = 0;
+    bool alive = true, need = true;         /* the same in the whole group */
+    int u[NC];
+    double rate = 0.0, time = 0.0, inf = 0.0;
+    uint64_t ctr = 0;
+    int err = 0, err_tr = -1;
+    double err_t = 0.0, err_rate = 0.0;
     unsigned nfired = 0;
     const double *v = nullptr, *ld = nullptr, *gd = nullptr;
     si_recip dc = si_recip_none();
     for (;;) {
-        const unsigned want = __ballot_sync(FULL, alive && need);
-        const bool holds_heavy = __any_sync(FULL, alive && !need && heavy);
-        const bool from_heavy = heavy_left;
-        if (want && !holds_heavy) {
-            const int leader = __ffs(want) - 1;
-            unsigned long long base = 0;
-            if (lane == leader)
-                base = atomicAdd(&s.queue_next[par * 2 + (from_heavy ? 0 : 1)],
-                                 (unsigned long long) __popc(want));
-            base = __shfl_sync(FULL, base, leader);
-            long long cand = -1;
-            bool empty = false;
+        /* groups without a node take the queue's next entries */
+        const unsigned want = __ballot_sync(FULL, alive && need && j == 0);
+        if (want) {
+            unsigned long long at = 0;
+            if (lane == __ffs((int) want) - 1)
+                at = atomicAdd(&s.queue_next[par * 2], (unsigned long long) __popc(want));
+            at = __shfl_sync(FULL, at, __ffs((int) want) - 1);
             if (alive && need) {
-                const unsigned long long pos = base + __popc(want & ((1u << lane) - 1u));
-                if (from_heavy) {
-                    if (pos < H) {
-                        int idx = (int) pos, c = 0;
-                        while (c < HEAVY_CLASSES - 1 && idx >= n[c]) {
-                            idx -= n[c];
-                            c++;
-                        }
-                        cand = s.heavy_list[(par * HEAVY_CLASSES + c) * MAX_HEAVY + idx];
-                    } else {
-                        empty = true;
+                unsigned long long pos = at + __popc(want & ((1u << base) - 1u));
+                long long cand = -1;
+                if (pos < H) {
+                    int idx = (int) pos, c = 0;
+                    while (c < HEAVY_CLASSES - 1 && idx >= n[c]) {
+                        idx -= n[c];
+                        c++;
                     }
-                } else if (pos >= Ntot) {
+                    cand = s.heavy_list[(par * HEAVY_CLASSES + c) * MAX_HEAVY + idx];
+                } else if (pos - H >= (unsigned long long) s.Ntot) {
                     alive = false;
-                } else if (s.heavy_mark[pos] != day + 1) {
-                    cand = (long long) pos;     /* heavy ones come from the heavy part */
+                } else if (H == 0 || s.heavy_mark[pos - H] != day + 1) {
+                    cand = (long long) (pos - H);
                 }
-            }
-            if (from_heavy && __any_sync(FULL, empty))
-                heavy_left = false;
-            if (cand >= 0) {
-                g = cand;
-                heavy = from_heavy;
-                const int node = node_of(s, g);
-                load_u<NC>(s.u + g * NC, a.u);
-#pragma unroll
-                for (int j = 0; j < NT; j++) {
-                    const size_t k = (size_t) j * s.Ntot + g;
-                    a.rate[j] = s.t_rate[k];
-                    a.time[j] = s.react_time[k];
-                    a.inf[j] = s.react_inf[k];
-                    a.ctr[j] = s.react_ctr[k];
+                if (cand >= 0) {
+                    g = cand;
+                    load_u<NC>(s.u + g * NC, u);
+                    const size_t k = (size_t) (own ? j : 0) * s.Ntot + g;
+                    rate = s.t_rate[k];
+                    time = s.react_time[k];
+                    inf = s.react_inf[k];
+                    ctr = s.react_ctr[k];
+                    v = s.vA + g * ND;
+                    ld = s.ldata + (size_t) node_of(s, g) * s.Nld;
+                    gd = gdata_of(s, g);
+                    dc = si_recip_none();
+                    err = 0;
+                    err_tr = -1;
+                    err_t = err_rate = 0.0;
+                    nfired = 0;
+                    need = false;
                 }
-                a.err = 0;
-                a.err_tr = -1;
-                a.err_t = 0.0;
-                a.err_rate = 0.0;
-                v = s.vA + g * ND;
-                ld = s.ldata + (size_t) node * s.Nld;
-                gd = gdata_of(s, g);
-                dc = si_recip_none();
-                nfired = 0;
-                need = false;
             }
         }
         if (!__any_sync(FULL, alive))
             break;
-        if (alive && !need) {
-            /* one event; a heavy warp has nothing else to do and runs its
-             * nodes' whole days in this loop */
-            bool done;
-            do
-                done = aem_step<M>(s, a, g, next, v, ld, gd, sS, sG, nfired, dc);
-            while (heavy && !done);
-            if (done) {
-                aem_finish<M>(s, a, g, day, tt, next);
-                fired += nfired;
-                need = true;
-                heavy = false;
+        /* the smallest event time, the lowest transition among equal ones;
+         * the comparisons are those of a scan from transition 0: a time that
+         * is not a number is passed over, and in place 0 it stays */
+        const uint64_t tb = si_double_bits(time);
+        int64_t key = si_isnan_bits(tb) ? (j == 0 ? INT64_MIN : INT64_MAX) : si_dkey(tb);
+        int tr = j;
+        if (!own)
+            key = INT64_MAX;
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+            const int64_t k2 = __shfl_xor_sync(FULL, key, o);
+            const int t2 = __shfl_xor_sync(FULL, tr, o);
+            if (k2 < key || (k2 == key && t2 < tr)) {
+                key = k2;
+                tr = t2;
             }
         }
+        const double t = __shfl_sync(FULL, time, base + tr);
+        const bool busy = alive && !need;
+        bool done = busy && (isinf(t) || t >= next);
+        bool bad = false;
+        double nr = 0.0;
+        if (busy && !done) {
+            if (++nfired > s.max_fired) {
+                err = ERR_TIMEOUT;
+                err_tr = tr;
+                err_t = t;
+                done = true;
+            } else {
+                int neg = 0;
+#pragma unroll
+                for (int c = 0; c < NC; c++) {
+                    const int x = sS[tr * NC + c];
+                    u[c] += x;
+                    neg |= (x != 0) & (u[c] < 0);
+                }
+                if (neg) {
+                    err = ERR_NEGATIVE_STATE;
+                    err_tr = tr;
+                    err_t = t;
+                    err_rate = 0.0;
+                }
+                if (own && (j == tr || ((sG[tr] >> j) & 1u))) {
+                    const double old = rate;
+#pragma unroll
+                    for (int k = 0; k < NT; k++)
+                        if (k == j)
+                            nr = M::rate(k, u, v, ld, gd, t, dc);
+                    rate = nr;
+                    bad = si_bad_rate(nr);
+                    aem_calc_times(time, inf, t, old, nr, s.seed, g, NT, j, ctr, &nl);
+                }
+            }
+        }
+        const unsigned bads = __ballot_sync(FULL, bad);
+        if (bads) {
+            /* the dependents are refreshed in order, the fired transition
+             * last: the last invalid rate is the one reported */
+            const unsigned mine = bads & group;
+            const int at = !mine ? lane
+                           : (mine >> (base + tr)) & 1u ? base + tr : 31 - __clz((int) mine);
+            const double r = __shfl_sync(FULL, nr, at);
+            if (mine) {
+                err = ERR_INVALID_RATE;
+                err_tr = at - base;
+                err_t = t;
+                err_rate = r;
+            }
+        }
+        if (done) {
+            /* the end of the node's day: its error, or its E1 events */
+            if (j == 0) {
+                if (err) {
+                    record_error(s, err, PHASE_SSA, day, g, err_tr, -1, err_t, err_rate);
+                } else {
+                    int2 at = s.e1_next[g];
+                    if (at.y == day) {
+                        si_rng r;
+                        uint64_t seed, sid;
+                        int e_code = 0, e_idx = -1;
+                        stream_key(s, g, seed, sid);
+                        si_rng_init(&r, seed, sid, s.ctr[g]);
+                        node_e1<NC>(s, u, at, node_of(s, g), day, r, e_code, e_idx);
+                        s.update[g] = 1;
+                        s.e1_next[g] = at;
+                        s.ctr[g] = r.ctr;
+                        if (e_code)
+                            record_error(s, e_code, PHASE_E1, day, g, -1, e_idx, tt, 0);
+                    }
+                }
+                store_u<NC>(s.u + g * NC, u);
+                s.t_time[g] = next;
+                fired += nfired;
+            }
+            if (own) {
+                const size_t k = (size_t) j * s.Ntot + g;
+                s.t_rate[k] = rate;
+                s.react_time[k] = time;
+                s.react_inf[k] = inf;
+                s.react_ctr[k] = ctr;
+            }
+            need = true;
+        }
+        __syncwarp();
     }
     add_fired(s, fired);
 }
@@ -3340,7 +3350,7 @@ struct Launch {
     }
     static cudaError_t aem_day(const DevState &s, int day, double tt, double next, cudaStream_t st)
     {
-        const long long need = (long long) blocks_for(s.Ntot, SSA_BLOCK);
+        const long long need = (long long) blocks_for(s.Ntot, SSA_BLOCK / AemLanes<M>::value);
         const int grid = (int) (need < aem_resident_blocks() ? need : aem_resident_blocks());
         return launch_day(s.chained, 1, k_aem_day<M>, grid, SSA_BLOCK, st, s, day, tt, next);
     }
