@@ -37,6 +37,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <tuple>
 #include <vector>
@@ -2609,12 +2610,16 @@ public:
         /* two threads: eight take three times as long, on the process's
          * memory map */
         const size_t n = std::min((size_t) 2, parts.size());
-        for (size_t t = 0; t < n; t++)
-            threads.emplace_back([this] {
-                for (size_t k = next++; k < parts.size(); k = next++)
-                    if (madvise(parts[k].first, parts[k].second, MADV_POPULATE_WRITE))
-                        return;
-            });
+        try {
+            for (size_t t = 0; t < n; t++)
+                threads.emplace_back([this] {
+                    for (size_t k = next++; k < parts.size(); k = next++)
+                        if (madvise(parts[k].first, parts[k].second, MADV_POPULATE_WRITE))
+                            return;
+                });
+        } catch (const std::system_error &) {
+            /* no thread to be had: the copy faults the pages in */
+        }
     }
     void join()
     {

@@ -1689,6 +1689,7 @@ __global__ void __launch_bounds__(256) k_quick(DevState s, int day, double tt, d
     const long long g = blockIdx.x * (long long) blockDim.x + threadIdx.x;
     bool listed = false;
     const float left = trunc_to_float(next - tt);
+    const float ulps = 1e-15f * fabsf((float) next);    /* of a time's rounding */
     day_begin();
     if (g < s.Ntot && load_flag(s.err_day) >= day && s.heavy_mark[g] != day + 1 &&
         !job_over(s, g, day)) {
@@ -1712,12 +1713,13 @@ __global__ void __launch_bounds__(256) k_quick(DevState s, int day, double tt, d
             philox_block(r, c >> 2, p0, p1, p2, p3);
             const uint32_t w = word_of(p0, p1, p2, p3, (uint32_t) c & 3u);
             /* -log(u) against the rate sum times the day's rest in single
-             * precision; where that is within its error of a tie (a few in
-             * 10^5), the quotient in double precision as the SSA forms it */
+             * precision; where that is within its error, or the times'
+             * rounding, of a tie (a few in 10^5), the quotient in double
+             * precision as the SSA forms it */
             const float L = -__logf(((float) w + 0.5f) * 2.3283064365386963e-10f);
-            const float x = trunc_to_float(sum) *
-                            (t == tt ? left : trunc_to_float(next - t));
-            const float slack = 1e-5f * (L + x) + 1e-5f;
+            const float fsum = trunc_to_float(sum);
+            const float x = fsum * (t == tt ? left : trunc_to_float(next - t));
+            const float slack = 1e-5f * (L + x) + 1e-5f + fsum * ulps;
             if (L > x + slack)
                 c += 1;                         /* the waiting time's draw was used */
             else if (L < x - slack)
