@@ -1590,6 +1590,8 @@ static cudaError_t launch_all(siminf_gpu_plan *p, DevState s, cudaStream_t st, K
 {
     const Launchers *L = p->L;
     const int ndays = p->max_days > 0 ? std::min(p->max_days, p->ndays) : p->ndays;
+    if (p->horizon)
+        s.heavy_rate = 0.0;             /* no work queue: k_init lists no heavy nodes */
     cudaError_t e = timed(kp, 0, st, [&] {
         return s.aem ? L->aem_init(s, p->tt0, st) : L->init(s, p->tt0, st);
     });
@@ -3208,10 +3210,9 @@ static int pf_session_create(const siminf_gpu_solver_args *a1, const siminf_gpu_
 /* Intervals g0 .. n_obs - 1 as replays of one CUDA graph, captured on the
  * session's first pass: the interval's seed, day schedule and observation
  * row are read from the device, and the finalize kernel moves the
- * interval counter on.  One replay: reset the state from the gathered
- * ancestors, k_init, k_horizon, weights, finalize (normalise, ESS,
- * resample), gather for the next interval.  Errors are read once, after
- * the last replay. */
+ * interval counter on.  One replay: k_init, k_horizon, weights, finalize
+ * (normalise, ESS, resample), the ancestors' state for the next interval.
+ * Errors are read once, after the last replay. */
 static int pf_session_graph(PfSession *ss, uint64_t seed, int prev_tlen)
 {
     siminf_gpu_plan *p = ss->p;
@@ -3238,12 +3239,24 @@ static int pf_session_graph(PfSession *ss, uint64_t seed, int prev_tlen)
     s.pf_seeds = ss->d_seeds;
     s.pf_days = ss->d_alldays;
     s.pf_days_stride = ss->nd;
+    s.heavy_rate = 0.0;                 /* no work queue: k_init lists no heavy nodes */
     const Launchers *L = p->L;
     const int Nn = s.Nn, Nc = s.Nc;
 
+    /* The ancestors' state goes straight where the interval's kernels read
+     * it: u and the first copy of v (the outputs it comes from are buffers
+     * of their own).  A post time step under rates that read t works in the
+     * second copy of v as well. */
+    auto gather = [&](int tlen, cudaStream_t st) {
+        cudaError_t r = pf_gather(s.U, s.V, tlen, (long long) ss->nu, (long long) ss->nv, ss->d_anc,
+                                  Np, s.u, s.vA, st);
+        if (r == cudaSuccess && s.Nd > 0 && !L->time_invariant)
+            r = cudaMemcpyAsync(s.vB, s.vA, (size_t) s.Ntot * s.Nd * sizeof(double),
+                                cudaMemcpyDeviceToDevice, st);
+        return r;
+    };
     /* the state of interval g0 from its ancestors, then the error flags */
-    e = pf_gather(s.U, s.V, prev_tlen, (long long) ss->nu, (long long) ss->nv, ss->d_anc, Np,
-                  p->d_u0, p->d_v0, pst);
+    e = gather(prev_tlen, pst);
     const int init_flags[3] = {0, INT_MAX, INT_MAX};
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(s.err_count, init_flags, sizeof(init_flags), cudaMemcpyHostToDevice,
@@ -3260,16 +3273,7 @@ static int pf_session_graph(PfSession *ss, uint64_t seed, int prev_tlen)
             e = cudaStreamBeginCapture(ss->gs, cudaStreamCaptureModeThreadLocal);
         if (e == cudaSuccess) {
             cudaStream_t gs = ss->gs;
-            cudaError_t c = cudaMemcpyAsync(s.u, p->d_u0, (size_t) s.Ntot * Nc * sizeof(int),
-                                            cudaMemcpyDeviceToDevice, gs);
-            if (c == cudaSuccess && s.Nd > 0)
-                c = cudaMemcpyAsync(s.vA, p->d_v0, (size_t) s.Ntot * s.Nd * sizeof(double),
-                                    cudaMemcpyDeviceToDevice, gs);
-            if (c == cudaSuccess && s.Nd > 0)
-                c = cudaMemcpyAsync(s.vB, p->d_v0, (size_t) s.Ntot * s.Nd * sizeof(double),
-                                    cudaMemcpyDeviceToDevice, gs);
-            if (c == cudaSuccess)
-                c = L->init(s, 0.0, gs);
+            cudaError_t c = L->init(s, 0.0, gs);
             if (c == cudaSuccess)
                 c = L->horizon(s, ss->d_alldays, ss->nd, gs);
             if (c == cudaSuccess)
@@ -3280,8 +3284,7 @@ static int pf_session_graph(PfSession *ss, uint64_t seed, int prev_tlen)
                                 ((uint64_t) 1) << 62, ss->d_anc, ss->d_anc_out, gs,
                                 ss->d_interval, ss->d_seeds + n_obs);
             if (c == cudaSuccess)
-                c = pf_gather(s.U, s.V, tl, (long long) ss->nu, (long long) ss->nv, ss->d_anc,
-                              Np, p->d_u0, p->d_v0, gs);
+                c = gather(tl, gs);
             e = cudaStreamEndCapture(gs, &graph);
             if (e == cudaSuccess)
                 e = c;
