@@ -200,7 +200,7 @@ int siminf_gpu_run_solver_mssm(siminf_gpu_solver_args *args,
  * at the start of a day reaches it are queued and simulated first, each by
  * a group of 8, 16 or 32 lanes (32 to a warp for models compiled from C
  * code; results are identical either way); 0 takes the default (0.5 below
- * 500,000 nodes in all replicates, 8 from there on and for compiled
+ * 500,000 nodes in all replicates, 4 from there on, 8 for compiled
  * models), a negative value turns the queue off.
  *
  * two_pass: a tuning knob, not a semantic option -- each day first
@@ -223,7 +223,8 @@ typedef struct siminf_gpu_options {
     int cap_transfers;
     int heavy_rate;     /* rate sum from which a node is queued first (0 = default, < 0 = off) */
     int gdata_per_replicate;
-    int two_pass;       /* > 0 on, < 0 off, 0 = on from 500,000 nodes (all replicates) */
+    int two_pass;       /* > 0 on, < 0 off, 0 = on from 200,000 nodes (all replicates;
+                         * 500,000 for compiled models) */
     int max_node_day_transitions;   /* > 0: the bound; 0: 2^28 */
     int streamed;       /* siminf_gpu_plan_create_ex: plan the events during the first run,
                          * beside the GPU, as the run entry points do (on host threads;

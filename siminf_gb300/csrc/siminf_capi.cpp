@@ -1300,12 +1300,13 @@ static int plan_create_impl(const siminf_gpu_solver_args *a, const siminf_gpu_mo
      * groups of lanes step the heavy nodes, a small model lists nearly all
      * its active nodes -- the chip has lanes to spare and a group's day is
      * shorter than a lane's (SISe3 of 1,600 nodes, 730 days: 29.9 ms at 0.5,
-     * 46.5 at 8; SEIR of 100,000, 180 days: 27.1 against 28.9) -- and a
-     * large one, whose ordinary nodes fill the chip, lists the long chains
-     * only (SEIR of 10^6, 240 days: 108.7 ms at 8, 115.1 at 1).  Models
-     * without lane groups: 8, the best of 2 to 128 on the 10^6-node SEIR
-     * workload. */
-    s.heavy_rate = L->lane_groups && Ntot < 500000 ? 0.5 : 8.0;
+     * 46.5 at 8; SEIR of 100,000, 180 days: 20.6 against 21.6 at 2) -- and a
+     * large one, whose ordinary nodes fill the chip, lists the longer chains
+     * only (SEIR of 10^6, 240 days: 87.8, 86.5, 87.1 ms at 2, 4, 8; 16
+     * replicates of 100,000, 150 days: 48.9, 48.4, 49.5; 700,000, 150 days:
+     * 32.8 at 0.5, 31.8 at 4).  Models without lane groups: 8, the best of 2
+     * to 128 on the 10^6-node SEIR workload. */
+    s.heavy_rate = !L->lane_groups ? 8.0 : Ntot < 500000 ? 0.5 : 4.0;
     if (const char *ev = getenv("SIMINF_HEAVY_RATE"))
         s.heavy_rate = atof(ev);
     if (opt && opt->heavy_rate > 0)
@@ -1320,10 +1321,13 @@ static int plan_create_impl(const siminf_gpu_solver_args *a, const siminf_gpu_mo
         if (!rc) rc = dalloc(&s.react_inf, (size_t) Ntot * Nt, own);
         if (!rc) rc = dalloc(&s.react_ctr, (size_t) Ntot * Nt, own);
     }
-    /* two-pass days (options, else SIMINF_TWO_PASS, else from 500,000
-     * nodes: below that a day is short and the extra launch costs more
-     * than the quiet nodes it takes out of the work queue) */
-    s.two_pass = Ntot >= 500000;
+    /* two-pass days (options, else SIMINF_TWO_PASS, else from 200,000
+     * nodes: below that a day is short and the extra launch costs more than
+     * the quiet nodes it takes out of the work queue -- SEIR, one pass
+     * against two: 150,000 nodes x 60 days 5.2 ms against 5.4, 200,000 x 180
+     * days 25.9 against 24.9, 300,000 x 150 days 22.5 against 21.6; models
+     * without lane groups from 500,000) */
+    s.two_pass = Ntot >= (L->lane_groups ? 200000 : 500000);
     if (const char *ev = getenv("SIMINF_TWO_PASS"))
         s.two_pass = atoi(ev) > 0;
     if (opt && opt->two_pass)
