@@ -3249,12 +3249,12 @@ static int pf_session_graph(PfSession *ss, uint64_t seed, int prev_tlen)
 
     /* The ancestors' state goes straight where the interval's kernels read
      * it: u and the first copy of v (the outputs it comes from are buffers
-     * of their own).  A post time step under rates that read t works in the
-     * second copy of v as well. */
+     * of their own).  Rates that read t, and a post time step that leaves
+     * entries of v_new alone, need the second copy of v as well. */
     auto gather = [&](int tlen, cudaStream_t st) {
         cudaError_t r = pf_gather(s.U, s.V, tlen, (long long) ss->nu, (long long) ss->nv, ss->d_anc,
                                   Np, s.u, s.vA, st);
-        if (r == cudaSuccess && s.Nd > 0 && !L->time_invariant)
+        if (r == cudaSuccess && s.Nd > 0 && !(L->time_invariant && L->pts_sets_v))
             r = cudaMemcpyAsync(s.vB, s.vA, (size_t) s.Ntot * s.Nd * sizeof(double),
                                 cudaMemcpyDeviceToDevice, st);
         return r;

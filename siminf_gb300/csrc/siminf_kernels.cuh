@@ -2825,6 +2825,19 @@ __device__ __forceinline__ int aem_pts_node(const DevState &s, long long g, int 
     return heavy_class<M>(s, sum);
 }
 
+/* M::pts() writes every entry of v_new, whatever the day: the shipped
+ * models.  The C code of a compiled model may leave an entry alone, which
+ * then holds the value of two days before: v and v_new are two buffers that
+ * change places at each day's end. */
+template <class M, class = void>
+struct model_pts_sets_v {
+    static constexpr bool value = M::ND == 0;
+};
+template <class M>
+struct model_pts_sets_v<M, decltype((void) M::PTS_SETS_V)> {
+    static constexpr bool value = M::PTS_SETS_V;
+};
+
 /* Every day of one node, for rates that ignore t: each pass of the loop is
  * one draw of a waiting time.  It ends in a transition or in the end of a
  * day, and both end in the same code: the rates at the new state (u after a
@@ -2850,10 +2863,15 @@ __device__ __forceinline__ void horizon_passes(const DevState &s, const DayInfo 
     const int rep = rep_of(s, g), node = node_of(s, g);
     const double *ld = s.ldata + (size_t) node * s.Nld;
     const double *gd = gdata_of(s, g);
-    double v[ND > 0 ? ND : 1];
+    /* v, and the other buffer's values where a post time step may keep some */
+    constexpr bool KEEPS = !model_pts_sets_v<M>::value;
+    double v[ND > 0 ? ND : 1], vo[ND > 0 ? ND : 1];
 #pragma unroll
-    for (int d = 0; d < ND; d++)
+    for (int d = 0; d < ND; d++) {
         v[d] = s.vA[g * ND + d];
+        if (KEEPS)
+            vo[d] = s.vB[g * ND + d];
+    }
     int2 e1;
     e1.x = s.e1_ptr[node];
     e1.y = e1.x < s.e1_ptr[node + 1] ? s.e1[e1.x].day : NO_E1;
@@ -2918,7 +2936,7 @@ __device__ __forceinline__ void horizon_passes(const DevState &s, const DayInfo 
         double vn[ND > 0 ? ND : 1];
 #pragma unroll
         for (int c = 0; c < ND; c++)
-            vn[c] = v[c];
+            vn[c] = KEEPS && kind == ENDS ? vo[c] : v[c];
         if (kind == ENDS) {
             if (draws)
                 ln.c += 1;                  /* the waiting time's draw was used */
@@ -3033,8 +3051,11 @@ __device__ __forceinline__ void horizon_passes(const DevState &s, const DayInfo 
             } else if (alive) {
                 store_columns<NC, ND>(s, rep, node, ln.u, vn, di.c0, di.c1);
 #pragma unroll
-                for (int c = 0; c < ND; c++)
+                for (int c = 0; c < ND; c++) {
+                    if (KEEPS)
+                        vo[c] = v[c];
                     v[c] = vn[c];
+                }
                 ln.fired = 0;
                 day_over = false;
                 d++;
@@ -3051,8 +3072,11 @@ __device__ __forceinline__ void horizon_passes(const DevState &s, const DayInfo 
     }
     if (mine) {
 #pragma unroll
-        for (int c = 0; c < ND; c++)
+        for (int c = 0; c < ND; c++) {
             s.vA[g * ND + c] = v[c];
+            if (KEEPS)
+                s.vB[g * ND + c] = vo[c];
+        }
     }
     r.ctr = ln.c;
 }
@@ -3366,8 +3390,8 @@ struct Launch {
     {
         static const Launchers t = {M::NC, M::NT, M::ND, M::NGD, M::PTS_LOCAL,
                                     M::RATES_TIME_INVARIANT, model_rates_total<M>::value,
-                                    init, horizon, quick, ssa_e1, e2_wave, pts_store,
-                                    aem_init, aem_day, aem_pts, e2_tail};
+                                    model_pts_sets_v<M>::value, init, horizon, quick, ssa_e1,
+                                    e2_wave, pts_store, aem_init, aem_day, aem_pts, e2_tail};
         return &t;
     }
 };

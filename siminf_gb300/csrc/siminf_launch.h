@@ -16,6 +16,7 @@ struct Launchers {
     bool pts_local;     /* post-time-step reads only its own node */
     bool time_invariant;    /* rates ignore t (the heavy part of the work queue applies) */
     bool lane_groups;       /* heavy nodes are stepped by groups of lanes */
+    bool pts_sets_v;        /* the post-time-step function writes every entry of v_new */
     cudaError_t (*init)(const DevState &s, double tt0, cudaStream_t st);
     cudaError_t (*horizon)(const DevState &s, const DayInfo *days, int ndays, cudaStream_t st);
     /* the first pass of a two-pass day (k_quick); ssa_e1 is the second */
@@ -55,7 +56,7 @@ const Launchers *launchers_for(const char *name);
  * the version with its own, which changes whenever the table or the device
  * state it passes changes layout. */
 #define SIMINF_MODEL_ABI \
-    (20261205 + (int) sizeof(siminf::DevState) + (int) sizeof(siminf::Launchers))
+    (20261206 + (int) sizeof(siminf::DevState) + (int) sizeof(siminf::Launchers))
 
 }  // namespace siminf
 

@@ -148,6 +148,7 @@ struct ModelSISe {
     static constexpr bool PTS_LOCAL = true;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
     static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
+    static constexpr bool PTS_SETS_V = true;   /* pts() writes all of v_new */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,
@@ -188,6 +189,7 @@ struct ModelSISe3 {
     static constexpr bool PTS_LOCAL = true;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
     static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
+    static constexpr bool PTS_SETS_V = true;   /* pts() writes all of v_new */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,
@@ -262,6 +264,7 @@ struct ModelSISe_sp {
     static constexpr bool PTS_LOCAL = false;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
     static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
+    static constexpr bool PTS_SETS_V = true;   /* pts() writes all of v_new */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,
@@ -302,6 +305,7 @@ struct ModelSISe3_sp {
     static constexpr bool PTS_LOCAL = false;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
     static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
+    static constexpr bool PTS_SETS_V = true;   /* pts() writes all of v_new */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,
@@ -366,6 +370,7 @@ struct ModelSISePF {
     static constexpr bool PTS_LOCAL = true;
     static constexpr bool RATES_TIME_INVARIANT = true;  /* rate() ignores t */
     static constexpr bool RATES_TOTAL = true;  /* rate() may see any non-negative u */
+    static constexpr bool PTS_SETS_V = true;   /* pts() writes all of v_new */
     template <class DC>
     __device__ __forceinline__ static double rate(int k, const int *u, const double *v,
                                                   const double *ldata, const double *gdata,
