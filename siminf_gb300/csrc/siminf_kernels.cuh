@@ -2942,7 +2942,10 @@ __device__ __forceinline__ void horizon_passes(const DevState &s, const DayInfo 
                 ln.c += 1;                  /* the waiting time's draw was used */
             else if (!day_over && !le_zero(si_double_bits(ln.sum)))
                 ln.err = ERR_INVALID_RATE;
-            ln.t = di.next;
+            /* the exact path sets the time itself: all rates zero under a
+             * positive sum leaves it at that step */
+            if (!day_over)
+                ln.t = di.next;
             fired += ln.fired;
             if (ln.err) {
                 record_error(s, ln.err, PHASE_SSA, d, g, -1, -1, tn, ln.sum);
