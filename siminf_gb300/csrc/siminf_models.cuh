@@ -12,13 +12,16 @@
  * The expressions, and their evaluation order, are those of the reference
  * model files (cited per model); the library is compiled with -fmad=false so
  * that no multiply-add is fused and every double rounds as it does in the
- * reference's C.  Four exact substitutions move work off GB300's slow FP64
+ * reference's C.  Three exact substitutions move work off GB300's slow FP64
  * pipe without changing a single bit of any result: int -> double
- * conversions are built from integer bits (si_i2d), a product with a count
- * is rounded from its integer digits (si_mul_i), a double sum of integer
+ * conversions are built from integer bits (si_i2d), a double sum of integer
  * counts that stays below 2^53 is formed as an integer sum and converted once
  * (every partial sum is exact either way), and divisions use si_div, an
- * IEEE round-to-nearest division on the integer pipes.  rate() takes a
+ * IEEE round-to-nearest division on the integer pipes.  Products stay on the
+ * FP64 pipe, but in SISe_sp's rates: its 30 or so integer instructions
+ * (si_mul_i) are a longer chain than one product (SIR, one node of 200,000:
+ * 351 ms with si_mul_i, 326 without; SEIR, 10^6 nodes x 240 days resident
+ * 86.9, 82.5; all-events, 100,000 nodes 36.7, 33.3).  rate() takes a
  * one-entry cache of the prepared divisor (si_div_cached): a population
  * count, which the transitions keep constant, is prepared once per change.
  * The cache is an si_recip, or in the SSA's speculative step an
@@ -45,10 +48,11 @@ struct ModelSIR {
         if (k == 0) {
             const long long n = (long long) u[0] + u[1] + u[2];     /* S_n + I_n + u[R] */
             /* the population divides every call: its reciprocal is cached */
-            const double q = si_div_cached(si_mul_i(si_mul_i(ldata[0], u[0]), u[1]), si_l2d(n > 0 ? n : 1), &dc);
+            const double q = si_div_cached(ldata[0] * si_i2d(u[0]) * si_i2d(u[1]),
+                                           si_l2d(n > 0 ? n : 1), &dc);
             return n > 0 ? q : 0.0;
         }
-        return si_mul_i(ldata[1], u[1]);
+        return ldata[1] * si_i2d(u[1]);
     }
     __device__ __forceinline__ static int pts(double *, const int *, const double *,
                                               const double *, const double *, int, double)
@@ -72,12 +76,13 @@ struct ModelSEIR {
         if (k == 0) {
             const long long n = (long long) u[0] + u[1] + u[2] + u[3];  /* S_n + u[E] + I_n + u[R] */
             /* the population divides every call: its reciprocal is cached */
-            const double q = si_div_cached(si_mul_i(si_mul_i(ldata[0], u[0]), u[2]), si_l2d(n > 0 ? n : 1), &dc);
+            const double q = si_div_cached(ldata[0] * si_i2d(u[0]) * si_i2d(u[2]),
+                                           si_l2d(n > 0 ? n : 1), &dc);
             return n > 0 ? q : 0.0;
         }
         if (k == 1)
-            return si_mul_i(ldata[1], u[1]);
-        return si_mul_i(ldata[2], u[2]);
+            return ldata[1] * si_i2d(u[1]);
+        return ldata[2] * si_i2d(u[2]);
     }
     __device__ __forceinline__ static int pts(double *, const int *, const double *,
                                               const double *, const double *, int, double)
@@ -101,10 +106,11 @@ struct ModelSIS {
         if (k == 0) {
             const long long n = (long long) u[0] + u[1];               /* S_n + I_n */
             /* the population divides every call: its reciprocal is cached */
-            const double q = si_div_cached(si_mul_i(si_mul_i(ldata[0], u[0]), u[1]), si_l2d(n > 0 ? n : 1), &dc);
+            const double q = si_div_cached(ldata[0] * si_i2d(u[0]) * si_i2d(u[1]),
+                                           si_l2d(n > 0 ? n : 1), &dc);
             return n > 0 ? q : 0.0;
         }
-        return si_mul_i(ldata[1], u[1]);
+        return ldata[1] * si_i2d(u[1]);
     }
     __device__ __forceinline__ static int pts(double *, const int *, const double *,
                                               const double *, const double *, int, double)
@@ -155,8 +161,8 @@ struct ModelSISe {
                                                   double t, DC &dc)
     {
         if (k == 0)
-            return si_mul_i(gdata[0] * v[0], u[0]);
-        return si_mul_i(gdata[1], u[1]);
+            return gdata[0] * v[0] * si_i2d(u[0]);
+        return gdata[1] * si_i2d(u[1]);
     }
     __device__ __forceinline__ static int pts(double *v_new, const int *u, const double *v,
                                               const double *ldata, const double *gdata,
@@ -169,7 +175,7 @@ struct ModelSISe {
                                               si_d2i(ldata[2]), si_d2i(ldata[3]), gdata[3],
                                               gdata[4], gdata[5], gdata[6]);
         if (n > 0)
-            v_new[0] += si_div(si_mul_i(gdata[2], u[1]), si_l2d(n)) + gdata[7];
+            v_new[0] += si_div(gdata[2] * si_i2d(u[1]), si_l2d(n)) + gdata[7];
         else
             v_new[0] += gdata[7];
         if (!isfinite(v_new[0]))
@@ -196,12 +202,12 @@ struct ModelSISe3 {
                                                   double t, DC &dc)
     {
         switch (k) {
-        case 0: return si_mul_i(gdata[0] * v[0], u[0]);
-        case 1: return si_mul_i(gdata[3], u[1]);
-        case 2: return si_mul_i(gdata[1] * v[0], u[2]);
-        case 3: return si_mul_i(gdata[4], u[3]);
-        case 4: return si_mul_i(gdata[2] * v[0], u[4]);
-        default: return si_mul_i(gdata[5], u[5]);
+        case 0: return gdata[0] * v[0] * si_i2d(u[0]);
+        case 1: return gdata[3] * si_i2d(u[1]);
+        case 2: return gdata[1] * v[0] * si_i2d(u[2]);
+        case 3: return gdata[4] * si_i2d(u[3]);
+        case 4: return gdata[2] * v[0] * si_i2d(u[4]);
+        default: return gdata[5] * si_i2d(u[5]);
         }
     }
     __device__ __forceinline__ static int pts(double *v_new, const int *u, const double *v,
@@ -216,7 +222,7 @@ struct ModelSISe3 {
                                               si_d2i(ldata[2]), si_d2i(ldata[3]), gdata[7],
                                               gdata[8], gdata[9], gdata[10]);
         if (n > 0)
-            v_new[0] += si_div(si_mul_i(gdata[6], I_n), si_l2d(n)) + gdata[11];
+            v_new[0] += si_div(gdata[6] * si_i2d(I_n), si_l2d(n)) + gdata[11];
         else
             v_new[0] += gdata[11];
         if (!isfinite(v_new[0]))
@@ -270,6 +276,8 @@ struct ModelSISe_sp {
                                                   const double *ldata, const double *gdata,
                                                   double t, DC &dc)
     {
+        /* off the FP64 pipe, which a day's groups of lanes fill on a grid
+         * (52 x 52 nodes x 120 days: 3.77 ms, 4.10 by si_i2d and a product) */
         if (k == 0)
             return si_mul_i(gdata[0] * v[0], u[0]);
         return si_mul_i(gdata[1], u[1]);
@@ -350,9 +358,9 @@ struct ModelSIRmparse {
     {
         if (k == 0) {
             const double N = si_i2d(u[0] + u[1] + u[2]);             /* int sum, as in C */
-            return si_div_cached(si_mul_i(si_mul_i(gdata[0], u[0]), u[1]), N, &dc);
+            return si_div_cached(gdata[0] * si_i2d(u[0]) * si_i2d(u[1]), N, &dc);
         }
-        return si_mul_i(gdata[1], u[1]);
+        return gdata[1] * si_i2d(u[1]);
     }
     __device__ __forceinline__ static int pts(double *, const int *, const double *,
                                               const double *, const double *, int, double)
@@ -377,8 +385,8 @@ struct ModelSISePF {
                                                   double t, DC &dc)
     {
         if (k == 0)
-            return si_mul_i(gdata[0] * v[0], u[0]);
-        return si_mul_i(gdata[1], u[1]);
+            return gdata[0] * v[0] * si_i2d(u[0]);
+        return gdata[1] * si_i2d(u[1]);
     }
     __device__ __forceinline__ static int pts(double *v_new, const int *u, const double *v,
                                               const double *ldata, const double *gdata,
@@ -388,7 +396,7 @@ struct ModelSISePF {
         const double phi = v[0];
         double x = phi * (1.0 - 0.03);
         if (n > 0)
-            x += si_div(si_mul_i(0.05, u[1]), si_l2d(n));
+            x += si_div(0.05 * si_i2d(u[1]), si_l2d(n));
         v_new[0] = x;
         return si_dne(phi, x);
     }
