@@ -2838,6 +2838,12 @@ struct model_pts_sets_v<M, decltype((void) M::PTS_SETS_V)> {
     static constexpr bool value = M::PTS_SETS_V;
 };
 
+/* A rate sum of 64 or more: a day of a lone chain, not of a node among many. */
+__device__ __forceinline__ bool busy_sum(double sum)
+{
+    return (unsigned) (si_double_bits(sum) >> 32) - 0x40500000u < 0x7FF00000u - 0x40500000u;
+}
+
 /* Every day of one node, for rates that ignore t: each pass of the loop is
  * one draw of a waiting time.  It ends in a transition or in the end of a
  * day, and both end in the same code: the rates at the new state (u after a
@@ -2848,9 +2854,15 @@ struct model_pts_sets_v<M, decltype((void) M::PTS_SETS_V)> {
  * a week of the particle filter's SISe, against about 21 passes.  What a
  * step meets rarely (a division off the integer path, a zero rate selected,
  * a negative state, an invalid rate, the transition bound) is redone on the
- * exact path, to the end of that day.  Every lane of the warp calls it;
- * `alive` says whether it has a node. */
-template <class M>
+ * exact path, to the end of that day.
+ * With BUSY, a warp whose every node fires 64 times a day or more (busy_sum)
+ * runs its nodes to the end of the day as ssa_run_day does: lanes at
+ * different days gain nothing there, and a draw a pass is a longer chain than
+ * a quarter of a batch of four.  Its test costs the other warps 1 to 3%
+ * (1,000 to 40,000 nodes of 100), and where warps are many a chain's latency
+ * is hidden, so it is for the smaller runs (Launch::horizon).
+ * Every lane of the warp calls it; `alive` says whether it has a node. */
+template <class M, bool BUSY>
 __device__ __forceinline__ void horizon_passes(const DevState &s, const DayInfo *days, int ndays,
                                                long long g, bool alive, SsaLane<M> &ln, si_rng &r,
                                                uint64_t &c_other, const int *sS,
@@ -2888,8 +2900,28 @@ __device__ __forceinline__ void horizon_passes(const DevState &s, const DayInfo 
     ln.q3 = 0;
     uint64_t have = ~0ULL;              /* the Philox block whose last word ln.q3 is */
     bool day_over = false;              /* the day ended on the exact path */
-    while (__any_sync(FULL, alive)) {
+    bool busy = false;                  /* a long day is ahead of the node */
+    for (;;) {
         enum { NONE, FIRES, ENDS, REDO };
+        if (__builtin_expect(!__any_sync(FULL, alive && !busy), 0)) {
+            if (!BUSY || !__any_sync(FULL, alive))
+                break;
+            /* every node here is busy: their days in batches of four draws */
+            if (alive) {
+                ln.err_tr = -1;
+                ln.err_t = 0.0;
+                ln.err_rate = 0.0;
+                ssa_run_day<M>(ln, r, di.next, v, ld, gd, sS, sG, s.max_fired, nl);
+                have = ~0ULL;
+                day_over = true;
+                if (ln.err) {
+                    record_error(s, ln.err, PHASE_SSA, d, g, ln.err_tr, -1, ln.err_t, ln.err_rate);
+                    fired += ln.fired;
+                    alive = false;
+                }
+            }
+            __syncwarp();
+        }
         int kind = alive ? ENDS : NONE;
         const bool draws = alive && !day_over && si_finite_pos(ln.sum);
         double L = 0.0, U = 0.0, tn = ln.t;
@@ -3034,6 +3066,7 @@ __device__ __forceinline__ void horizon_passes(const DevState &s, const DayInfo 
                 ;
             have = ~0ULL;
             day_over = true;
+            busy = false;
             if (ln.err) {
                 record_error(s, ln.err, PHASE_SSA, d, g, ln.err_tr, -1, ln.err_t, ln.err_rate);
                 fired += ln.fired;
@@ -3051,7 +3084,9 @@ __device__ __forceinline__ void horizon_passes(const DevState &s, const DayInfo 
                 ln.t = tn;
                 ln.c += 2;
                 ln.fired++;
+                busy = BUSY && busy_sum(sum2);
             } else if (alive) {
+                busy = false;
                 store_columns<NC, ND>(s, rep, node, ln.u, vn, di.c0, di.c1);
 #pragma unroll
                 for (int c = 0; c < ND; c++) {
@@ -3087,7 +3122,7 @@ __device__ __forceinline__ void horizon_passes(const DevState &s, const DayInfo 
 /* Whole horizon of one (replicate, node) in one thread: valid when no
  * external transfer couples nodes and the post-time-step function reads
  * only its own node. */
-template <class M>
+template <class M, bool BUSY>
 __global__ void __launch_bounds__(HORIZON_BLOCK, M::NT <= 4 ? 4 : 2)
 k_horizon(DevState s, const DayInfo *days, int ndays, int lanes)
 {
@@ -3128,7 +3163,7 @@ k_horizon(DevState s, const DayInfo *days, int ndays, int lanes)
         }
     }
     if constexpr (M::RATES_TIME_INVARIANT) {
-        horizon_passes<M>(s, days, ndays, g, have, ln, r, c_other, sS, sG, &nl, fired);
+        horizon_passes<M, BUSY>(s, days, ndays, g, have, ln, r, c_other, sS, sG, &nl, fired);
     } else if (have) {
         const int rep = rep_of(s, g), node = node_of(s, g);
         double *v = s.vA + g * ND, *vn = s.vB + g * ND;
@@ -3283,8 +3318,18 @@ struct Launch {
         int lanes = 32;
         while (lanes > 1 && (s.Ntot + lanes / 2 - 1) / (lanes / 2) <= 4ll * sm_count())
             lanes /= 2;
-        k_horizon<M><<<blocks_for(s.Ntot, lanes * (HORIZON_BLOCK / 32)), HORIZON_BLOCK, 0, st>>>(
-            s, days, ndays, lanes);
+        const unsigned grid = blocks_for(s.Ntot, lanes * (HORIZON_BLOCK / 32));
+        /* up to four warps a scheduler, busy days in batches of four draws
+         * (SIR, nodes of 3,000 x 40 days: 40,000 nodes 12.5 ms without, 11.8
+         * with; 80,000 22.3, 21.3; 160,000 35.3, 37.3; one node of 200,000 x
+         * 60 days 326, 206) */
+        if constexpr (M::RATES_TIME_INVARIANT) {
+            if (s.Ntot <= 4 * 32 * 4ll * sm_count()) {
+                k_horizon<M, true><<<grid, HORIZON_BLOCK, 0, st>>>(s, days, ndays, lanes);
+                return cudaGetLastError();
+            }
+        }
+        k_horizon<M, false><<<grid, HORIZON_BLOCK, 0, st>>>(s, days, ndays, lanes);
         return cudaGetLastError();
     }
     /* k_ssa_e1 is persistent: as many blocks as can be resident at once
