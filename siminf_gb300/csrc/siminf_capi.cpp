@@ -122,6 +122,40 @@ int upload(T **p, const T *src, size_t n, std::vector<void *> &owned, cudaStream
     return 0;
 }
 
+/* Column c of E as a set of compartments, with ECOL_PLAIN where that is all
+ * a sample needs (DevState::ecol); 0 otherwise. */
+uint32_t column_set(const siminf_gpu_solver_args *a, int c)
+{
+    uint32_t rows = ECOL_PLAIN;
+    for (int k = a->jcE[c]; k < a->jcE[c + 1]; k++) {
+        const int row = a->irE[k];
+        if (row < 0 || row >= std::min(a->Nc, (int) MAX_NC) ||
+            (k > a->jcE[c] && (row <= a->irE[k - 1] || a->prE[k] != a->prE[k - 1])))
+            return 0;
+        rows |= 1u << row;
+    }
+    return rows;
+}
+
+/* Whether e2_apply samples most of the schedule's transfers itself, by up to
+ * 128 events spread over the table: sizes given as counts, unshifted, from
+ * plain columns (among the first max_select, whose E is known). */
+bool plain_transfers(const siminf_gpu_solver_args *a, int max_select)
+{
+    enum { LOOKS = 128 };
+    int transfers = 0, others = 0;
+    for (int k = 0; k < std::min(a->len, (int) LOOKS); k++) {
+        const long long i = (long long) a->len * k / std::min(a->len, (int) LOOKS);
+        if (a->event[i] != SIMINF_GPU_EXTERNAL_TRANSFER_EVENT)
+            continue;
+        const int sel = a->select[i];
+        transfers++;
+        others += a->n[i] <= 0 || a->shift[i] > 0 ||
+                  (sel > 0 && sel <= max_select && !column_set(a, sel - 1));
+    }
+    return 8 * others <= transfers;
+}
+
 /* The first ncol columns of E on the device: the sparse matrix, and per
  * column the compartments it selects from as a set (DevState::ecol). */
 int upload_E(DevState &s, const siminf_gpu_solver_args *a, int ncol, std::vector<void *> &owned,
@@ -129,18 +163,8 @@ int upload_E(DevState &s, const siminf_gpu_solver_args *a, int ncol, std::vector
 {
     const int nnz = a->jcE[ncol];
     std::vector<uint32_t> cols((size_t) std::max(ncol, 1), 0u);
-    for (int c = 0; c < ncol; c++) {
-        uint32_t rows = 0;
-        bool plain = true;
-        for (int k = a->jcE[c]; k < a->jcE[c + 1]; k++) {
-            const int row = a->irE[k];
-            plain = plain && row >= 0 && row < std::min(a->Nc, (int) MAX_NC) &&
-                    (k == a->jcE[c] || (row > a->irE[k - 1] && a->prE[k] == a->prE[k - 1]));
-            if (plain)
-                rows |= 1u << row;
-        }
-        cols[c] = plain ? rows | ECOL_PLAIN : 0u;
-    }
+    for (int c = 0; c < ncol; c++)
+        cols[c] = column_set(a, c);
     int *djc, *dir;
     double *dpr;
     uint32_t *dcol;
@@ -1245,6 +1269,7 @@ static int plan_create_impl(const siminf_gpu_solver_args *a, const siminf_gpu_mo
          * schedule scan found both). */
         const int maxsel = p->max_select, maxshift = p->max_shift;
         rc = upload_E(s, a, maxsel, own, st);
+        p->e2_plain = plain_transfers(a, maxsel);
         /* N is "defined" whenever the caller passes it (src/SimInf.c:302-305),
          * even if no event shifts. */
         s.hasN = a->N != nullptr;
@@ -1544,14 +1569,20 @@ static cudaError_t download_columns(const siminf_gpu_plan *p, const siminf_gpu_s
 /* The wavefronts of one day: offsets into d_e2 and event counts.  The
  * last ones, while each holds at most E2_TAIL_ITEMS events x replicates,
  * run together in one cluster (k_e2_tail), up to E2_TAIL_WAVES per launch;
- * the others, one launch each. */
+ * the others, one launch each.  Proportions and weighted columns sample in
+ * double precision and shifts go round by memory (e2_apply_any): eight SMs
+ * are too few for a wave of those, and the cluster takes none of more than a
+ * block's (SEIR, 20,000 nodes x 60 days, 10,000 transfers a day: proportions
+ * 32.7 ms with 8,192, 27.2 with 2,048, 24.1 with 512; weighted columns 9.3,
+ * 8.7, 8.5; shifts 8.4, 8.0, 8.0). */
 static cudaError_t launch_day_waves(const siminf_gpu_plan *p, const DevState &s,
                                     const long long *off, const long long *cnt, int nw, int d,
                                     double tt, cudaStream_t st, KernelProfile *kp)
 {
     const Launchers *L = p->L;
+    const long long most = p->e2_plain ? E2_TAIL_ITEMS : E2_BLOCK_ITEMS;
     int t = nw;
-    while (t > 0 && cnt[t - 1] * (long long) s.Nrep <= E2_TAIL_ITEMS)
+    while (t > 0 && cnt[t - 1] * (long long) s.Nrep <= most)
         t--;
     if (nw - t < 2)
         t = nw;                         /* a single small wave: its own launch */
@@ -1848,6 +1879,7 @@ static cudaError_t launch_streamed(siminf_gpu_plan *p, DevState s, cudaStream_t 
                 s.prE = p->s.prE;
                 s.ecol = p->s.ecol;
                 p->max_select = msel;
+                p->e2_plain = plain_transfers(a, msel);
             }
             if (mshift > p->max_shift && a->N) {
                 int *dN;
@@ -2373,6 +2405,7 @@ static cudaError_t launch_streamed_dev(siminf_gpu_plan *p, DevState s, cudaStrea
             s.prE = p->s.prE;
             s.ecol = p->s.ecol;
             p->max_select = pl.ch.max_select;
+            p->e2_plain = plain_transfers(a, p->max_select);
         }
         if (pl.ch.max_shift > p->max_shift && a->N) {
             int *dN;
