@@ -1971,10 +1971,13 @@ __global__ void __launch_bounds__(SSA_BLOCK, MINB) k_ssa_e1(DevState s, int day,
 /* One external transfer of one replicate (src/solvers/SimInf_solver.c:
  * 824-902): sample from the source, add to the destination (atomics: adds
  * into one destination commute within a wavefront), subtract from the
- * source (exclusive to this event within its wavefront).  Any transfer;
- * out of line behind e2_apply, which handles the common ones. */
+ * source (exclusive to this event within its wavefront).  Any transfer,
+ * behind e2_apply, which handles the common ones; inlined, as a call costs
+ * the waves of both kinds (SISe3, 10,000 nodes x 60 days of proportions 4.95 ms
+ * of waves called, 4.18 inlined; SEIR, 20,000 nodes x 120 days of counts 3.58,
+ * 3.29). */
 template <class M>
-__device__ __noinline__ void e2_apply_any(const DevState &s, const E2Rec &e, int rep, int day,
+__device__ __forceinline__ void e2_apply_any(const DevState &s, const E2Rec &e, int rep, int day,
                                           double tt)
 {
     constexpr int NC = M::NC;
