@@ -2552,8 +2552,13 @@ struct AemLanes {
  * each refresh their own rate and time, side by side: one division a step
  * where one lane did NT of them one after the other.  Bound: the busiest
  * node's chain.  SEIR, 100,000 nodes x 120 days: 50.3 ms with a lane a node,
- * 26.3 with four. */
-template <class M>
+ * 26.3 with four.
+ * With WIDE, for many nodes a group (Launch::aem_day), a warp looks through
+ * the ordinary part 32 nodes at a time, a lane a node: one whose event times
+ * all pass the day's end, and without an E1 event, is done, and the groups
+ * take the others.  Handed out a group a node, a day of 500,000 nodes without
+ * an infected one took 55 us, 25 with a lane a node, and takes 20. */
+template <class M, bool WIDE>
 __global__ void __launch_bounds__(SSA_BLOCK, 4) k_aem_day(DevState s, int day, double tt,
                                                           double next)
 {
@@ -2596,47 +2601,92 @@ __global__ void __launch_bounds__(SSA_BLOCK, 4) k_aem_day(DevState s, int day, d
     unsigned nfired = 0;
     const double *v = nullptr, *ld = nullptr, *gd = nullptr;
     si_recip dc = si_recip_none();
+    /* WIDE, the same in the whole warp: the heavy part and the ordinary one
+     * may have entries; the lanes whose `mine` is a node to hand out */
+    bool heavy_left = H > 0, more = true;
+    unsigned listed = 0;
+    long long mine = 0;
     for (;;) {
         /* groups without a node take the queue's next entries */
         const unsigned want = __ballot_sync(FULL, alive && need && j == 0);
         if (want) {
-            unsigned long long at = 0;
-            if (lane == __ffs((int) want) - 1)
-                at = atomicAdd(&s.queue_next[par * 2], (unsigned long long) __popc(want));
-            at = __shfl_sync(FULL, at, __ffs((int) want) - 1);
-            if (alive && need) {
-                unsigned long long pos = at + __popc(want & ((1u << base) - 1u));
-                long long cand = -1;
-                if (pos < H) {
-                    int idx = (int) pos, c = 0;
-                    while (c < HEAVY_CLASSES - 1 && idx >= n[c]) {
-                        idx -= n[c];
-                        c++;
+            const unsigned place = __popc(want & ((1u << base) - 1u));  /* the group's among them */
+            long long cand = -1;
+            if (!WIDE || heavy_left) {
+                unsigned long long at = 0;
+                if (lane == __ffs((int) want) - 1)
+                    at = atomicAdd(&s.queue_next[par * 2], (unsigned long long) __popc(want));
+                at = __shfl_sync(FULL, at, __ffs((int) want) - 1);
+                heavy_left = at + __popc(want) < H;
+                if (alive && need) {
+                    const unsigned long long pos = at + place;
+                    if (pos < H) {
+                        int idx = (int) pos, c = 0;
+                        while (c < HEAVY_CLASSES - 1 && idx >= n[c]) {
+                            idx -= n[c];
+                            c++;
+                        }
+                        cand = s.heavy_list[(par * HEAVY_CLASSES + c) * MAX_HEAVY + idx];
+                    } else if (!WIDE) {
+                        if (pos - H >= (unsigned long long) s.Ntot)
+                            alive = false;
+                        else if (H == 0 || s.heavy_mark[pos - H] != day + 1)
+                            cand = (long long) (pos - H);
                     }
-                    cand = s.heavy_list[(par * HEAVY_CLASSES + c) * MAX_HEAVY + idx];
-                } else if (pos - H >= (unsigned long long) s.Ntot) {
-                    alive = false;
-                } else if (H == 0 || s.heavy_mark[pos - H] != day + 1) {
-                    cand = (long long) (pos - H);
                 }
-                if (cand >= 0) {
-                    g = cand;
-                    load_u<NC>(s.u + g * NC, u);
-                    const size_t k = (size_t) (own ? j : 0) * s.Ntot + g;
-                    rate = s.t_rate[k];
-                    time = s.react_time[k];
-                    inf = s.react_inf[k];
-                    ctr = s.react_ctr[k];
-                    v = s.vA + g * ND;
-                    ld = s.ldata + (size_t) node_of(s, g) * s.Nld;
-                    gd = gdata_of(s, g);
-                    dc = si_recip_none();
-                    err = 0;
-                    err_tr = -1;
-                    err_t = err_rate = 0.0;
-                    nfired = 0;
-                    need = false;
+            } else {
+                while (!listed && more) {
+                    unsigned long long at = 0;
+                    if (lane == 0)
+                        at = atomicAdd(&s.queue_next[par * 2 + 1], 32ull);
+                    at = __shfl_sync(FULL, at, 0);
+                    more = at + 32 < (unsigned long long) s.Ntot;
+                    mine = (long long) at + lane;
+                    bool take = mine < s.Ntot && (H == 0 || s.heavy_mark[mine] != day + 1);
+                    if (take) {
+                        double t = s.react_time[mine];
+#pragma unroll
+                        for (int k = 1; k < NT; k++) {
+                            const double x = s.react_time[(size_t) k * s.Ntot + mine];
+                            if (x < t)
+                                t = x;
+                        }
+                        if ((isinf(t) || t >= next) && s.e1_next[mine].y != day) {
+                            s.t_time[mine] = next;
+                            take = false;
+                        }
+                    }
+                    listed = __ballot_sync(FULL, take);
                 }
+                /* the k-th group takes the k-th node of the list */
+                const unsigned from = __fns(listed, 0, (int) place + 1);
+                const unsigned last = __fns(listed, 0, __popc(want));
+                const long long c = __shfl_sync(FULL, mine, (int) (from & 31u));
+                if (alive && need) {
+                    if (from < 32)
+                        cand = c;
+                    else if (!more)
+                        alive = false;
+                }
+                listed = last < 32 ? listed & ~((2u << last) - 1u) : 0u;
+            }
+            if (cand >= 0) {
+                g = cand;
+                load_u<NC>(s.u + g * NC, u);
+                const size_t k = (size_t) (own ? j : 0) * s.Ntot + g;
+                rate = s.t_rate[k];
+                time = s.react_time[k];
+                inf = s.react_inf[k];
+                ctr = s.react_ctr[k];
+                v = s.vA + g * ND;
+                ld = s.ldata + (size_t) node_of(s, g) * s.Nld;
+                gd = gdata_of(s, g);
+                dc = si_recip_none();
+                err = 0;
+                err_tr = -1;
+                err_t = err_rate = 0.0;
+                nfired = 0;
+                need = false;
             }
         }
         if (!__any_sync(FULL, alive))
@@ -3413,23 +3463,36 @@ struct Launch {
         k_aem_init<M><<<blocks_for(s.Ntot, 256), 256, 0, st>>>(s, tt0);
         return cudaGetLastError();
     }
+    template <bool WIDE>
     static int aem_resident_blocks()
     {
         static int blocks = 0;
         if (!blocks) {
-            int dev = 0, nsm = 1, per = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_aem_day<M>, SSA_BLOCK, 0);
-            blocks = nsm * (per > 0 ? per : 1);
+            int per = 0;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_aem_day<M, WIDE>, SSA_BLOCK, 0);
+            blocks = sm_count() * (per > 0 ? per : 1);
         }
         return blocks;
     }
-    static cudaError_t aem_day(const DevState &s, int day, double tt, double next, cudaStream_t st)
+    template <bool WIDE>
+    static cudaError_t aem_day_with(const DevState &s, int day, double tt, double next,
+                                    cudaStream_t st)
     {
         const long long need = (long long) blocks_for(s.Ntot, SSA_BLOCK / AemLanes<M>::value);
-        const int grid = (int) (need < aem_resident_blocks() ? need : aem_resident_blocks());
-        return launch_day(s.chained, 1, k_aem_day<M>, grid, SSA_BLOCK, st, s, day, tt, next);
+        const int resident = aem_resident_blocks<WIDE>();
+        const int grid = (int) (need < resident ? need : resident);
+        return launch_day(s.chained, 1, k_aem_day<M, WIDE>, grid, SSA_BLOCK, st, s, day, tt, next);
+    }
+    static cudaError_t aem_day(const DevState &s, int day, double tt, double next, cudaStream_t st)
+    {
+        /* from eight nodes a resident group, quiet ones are looked through by
+         * lanes (SEIR of 1% infected nodes, 10^6 x 20 days 9.8 ms without, 8.3
+         * with; 300,000 x 30 5.6, 5.1; at five nodes a group SIS, 200,000 x 40,
+         * 3.9, 4.1) */
+        const long long groups =
+            (long long) aem_resident_blocks<true>() * (SSA_BLOCK / AemLanes<M>::value);
+        return s.Ntot >= 8 * groups ? aem_day_with<true>(s, day, tt, next, st)
+                                    : aem_day_with<false>(s, day, tt, next, st);
     }
     static cudaError_t aem_pts(const DevState &s, int day, double tt, int c0, int c1,
                                const double *v_in, double *v_out, cudaStream_t st)
