@@ -482,14 +482,16 @@ int siminf_gpu_plan_stats(const siminf_gpu_plan *plan, siminf_gpu_stats *out);
  * with one-pass and with two-pass days (siminf_gpu_options.two_pass).
  * Stage 2, from the best of stage 1: the SSA kernel's other register
  * budget (ssa_variant 1: more registers a thread, fewer resident warps),
- * then, for a plan of one model and one replicate with the heavy part on,
- * 8 lanes a warp for the heaviest class (heavy_lanes; 32 otherwise).  Stage 3, for plans with external transfers: the wavefront kernel's block
+ * then, for a plan of one model and one replicate with the heavy part on and
+ * a model compiled from C code, 8 lanes a warp for the heaviest class
+ * (heavy_lanes; 32 otherwise), then the layout the plan was created with.
+ * Stage 3, for plans with external transfers: the wavefront kernel's block
  * of 128 and 512 threads (256 otherwise).  The three fastest are then
  * timed again as repeated runs execute them (the third run of each, which
  * replays the run's CUDA graph), and their times replace the probes'; the
  * fastest of those is kept.  The choice is kept per device
- * model and size class (node count and day count to a power of two,
- * transfers or not): a later plan of the same class takes it without
+ * model, size class (node count and day count to a power of two,
+ * transfers or not) and created layout: a later plan of the same takes it without
  * probing (cached = 1; probe_days < 0 forces a new search).  Results never
  * depend on the layout; only the order in which nodes are simulated does.
  */

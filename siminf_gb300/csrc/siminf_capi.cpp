@@ -1359,6 +1359,8 @@ static int plan_create_impl(const siminf_gpu_solver_args *a, const siminf_gpu_mo
         s.two_pass = opt->two_pass > 0;
     if (s.aem)
         s.two_pass = 0;                 /* the work queue is the direct method's */
+    p->own = {s.heavy_rate, s.two_pass, s.ssa_variant,
+              s.wave_block == 256 || s.wave_block == 512 ? s.wave_block : 128, s.heavy_lanes};
     if (!rc) rc = dalloc(&s.active, (size_t) Ntot, own);
     if (!rc) {
         s.err_day = s.err_count + 1;
@@ -2780,14 +2782,19 @@ int siminf_gpu_plan_run(siminf_gpu_plan *p, void *cuda_stream)
     return plan_run_impl(p, (cudaStream_t) cuda_stream, nullptr);
 }
 
-/* The autotuner's choices, kept per device model and size class. */
+/* The autotuner's choices, kept per device model, size class and the layout
+ * the plan was created with, which is one of the candidates. */
 struct TuneKey {
     const Launchers *L;
     int nodes_class, days_class, transfers, aem, probe_days;
+    siminf_gpu_plan::Layout own;
     bool operator<(const TuneKey &o) const
     {
-        return std::tie(L, nodes_class, days_class, transfers, aem, probe_days) <
-               std::tie(o.L, o.nodes_class, o.days_class, o.transfers, o.aem, o.probe_days);
+        return std::tie(L, nodes_class, days_class, transfers, aem, probe_days, own.heavy_rate,
+                        own.two_pass, own.ssa_variant, own.wave_block, own.heavy_lanes) <
+               std::tie(o.L, o.nodes_class, o.days_class, o.transfers, o.aem, o.probe_days,
+                        o.own.heavy_rate, o.own.two_pass, o.own.ssa_variant, o.own.wave_block,
+                        o.own.heavy_lanes);
     }
 };
 static std::mutex g_tune_mu;
@@ -2812,7 +2819,7 @@ int siminf_gpu_plan_tune(siminf_gpu_plan *p, void *cuda_stream, int probe_days,
     const int want_days = probe_days < 0 ? -probe_days : probe_days;
     const int pdays = std::min(want_days > 0 ? want_days : 16, p->ndays);
     const TuneKey key{p->L, log2_class(p->s.Ntot), log2_class(p->ndays), p->e2_count > 0,
-                      p->s.aem, pdays};
+                      p->s.aem, pdays, p->own};
     auto apply = [&](const siminf_gpu_tune_result &r, int k) {
         p->s.heavy_rate = r.heavy_rate[k];
         p->s.two_pass = r.two_pass[k];
@@ -2867,15 +2874,15 @@ int siminf_gpu_plan_tune(siminf_gpu_plan *p, void *cuda_stream, int probe_days,
      * against 2.76 s with 32) */
     if (!rc && best >= 0 && !p->s.aem)
         probe(r.heavy_rate[best], r.two_pass[best], 1, 256, 0);
-    if (p->L->lane_groups) {
-        /* heavy nodes have groups of lanes, whatever heavy_lanes says: the
-         * probe is of the plan's own threshold, where it is below all others */
-        if (!rc && best >= 0 && !p->s.aem && saved > 0.0 && saved < cand[1])
-            probe(saved, r.two_pass[best], r.ssa_variant[best], 256, 8);
-    } else if (!rc && best >= 0 && !p->s.aem && r.heavy_rate[best] > 0.0 &&
-               p->L->time_invariant && p->s.Nrep == 1 && !p->s.job_of) {
+    if (!rc && best >= 0 && !p->s.aem && !p->L->lane_groups && r.heavy_rate[best] > 0.0 &&
+        p->L->time_invariant && p->s.Nrep == 1 && !p->s.job_of)
         probe(r.heavy_rate[best], r.two_pass[best], r.ssa_variant[best], 256, 8);
-    }
+    /* the layout the plan was created with: what tuning replaces is measured
+     * too (for models with lane groups, whose heavy_lanes nothing reads, in
+     * the place and with the 8 of the probe above) */
+    if (!rc && best >= 0)
+        probe(p->own.heavy_rate, p->own.two_pass, p->own.ssa_variant, p->own.wave_block,
+              p->L->lane_groups && !p->s.aem ? 8 : p->own.heavy_lanes);
     /* stage 3: the wavefront block */
     if (!rc && best >= 0 && p->e2_count > 0) {
         const siminf_gpu_tune_result b = r;

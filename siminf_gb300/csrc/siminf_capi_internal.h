@@ -63,6 +63,13 @@ struct siminf_gpu_plan {
     double *d_v0 = nullptr;
     double tt0 = 0;
 
+    /* The launch layout the plan was created with (the autotuner has its
+     * choice in s). */
+    struct Layout {
+        double heavy_rate = 0.0;
+        int two_pass = 0, ssa_variant = 0, wave_block = 0, heavy_lanes = 0;
+    } own;
+
     siminf_gpu_stats stats{};
     bool ran = false;
     int days_cap = 0;
