@@ -26,6 +26,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -246,8 +247,13 @@ extern "C" int siminf_gpu_run_batch(siminf_gpu_batch_job *jobs, int njobs,
                 f(k);
         };
         std::vector<std::thread> th;
-        for (int t = 1; t < nthreads; t++)
-            th.emplace_back(work);
+        th.reserve(nthreads);
+        try {
+            for (int t = 1; t < nthreads; t++)
+                th.emplace_back(work);
+        } catch (const std::system_error &) {
+            /* no more threads to be had: those there are do it all */
+        }
         work();
         for (auto &x : th)
             x.join();

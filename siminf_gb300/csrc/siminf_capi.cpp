@@ -488,15 +488,23 @@ static int threads_for(long long items)
     return (int) std::min((long long) planner_threads(), items / 16384 + 1);
 }
 
-/* Run f(t, n) on n = threads_for(items) threads and join. */
+/* Run f(t, n) for t = 0 .. n - 1, n = threads_for(items), a thread each, and
+ * join; the shares that no thread is to be had for run here. */
 template <class F>
 static void parallel(long long items, F &&f)
 {
-    const unsigned n = (unsigned) threads_for(items);
+    const int n = threads_for(items);
     std::vector<std::thread> th;
-    for (unsigned t = 1; t < n; t++)
-        th.emplace_back([&f, t, n] { f((int) t, (int) n); });
-    f(0, (int) n);
+    th.reserve(n);
+    int t = 1;
+    try {
+        for (; t < n; t++)
+            th.emplace_back([&f, t, n] { f(t, n); });
+    } catch (const std::system_error &) {
+        for (; t < n; t++)
+            f(t, n);
+    }
+    f(0, n);
     for (auto &x : th)
         x.join();
 }
@@ -2647,7 +2655,6 @@ public:
     }
     void start()
     {
-        const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
         /* two threads: eight take three times as long, on the process's
          * memory map */
         const size_t n = std::min((size_t) 2, parts.size());
@@ -2658,7 +2665,7 @@ public:
                         if (madvise(parts[k].first, parts[k].second, MADV_POPULATE_WRITE))
                             return;
                 });
-        } catch (const std::system_error &) {
+        } catch (const std::exception &) {
             /* no thread to be had: the copy faults the pages in */
         }
     }
