@@ -158,11 +158,13 @@ bool plain_transfers(const siminf_gpu_solver_args *a, int max_select)
 
 /* The first ncol columns of E on the device: the sparse matrix, and per
  * column the compartments it selects from as a set (DevState::ecol). */
-int upload_E(DevState &s, const siminf_gpu_solver_args *a, int ncol, std::vector<void *> &owned,
-             cudaStream_t st)
+int upload_E(siminf_gpu_plan *p, const siminf_gpu_solver_args *a, int ncol, cudaStream_t st)
 {
+    DevState &s = p->s;
+    std::vector<void *> &owned = p->owned;
     const int nnz = a->jcE[ncol];
-    std::vector<uint32_t> cols((size_t) std::max(ncol, 1), 0u);
+    p->ecols.emplace_back((size_t) std::max(ncol, 1), 0u);
+    std::vector<uint32_t> &cols = p->ecols.back();
     for (int c = 0; c < ncol; c++)
         cols[c] = column_set(a, c);
     int *djc, *dir;
@@ -1276,7 +1278,7 @@ static int plan_create_impl(const siminf_gpu_solver_args *a, const siminf_gpu_mo
          * the events use (the struct carries no column counts; the
          * schedule scan found both). */
         const int maxsel = p->max_select, maxshift = p->max_shift;
-        rc = upload_E(s, a, maxsel, own, st);
+        rc = upload_E(p, a, maxsel, st);
         p->e2_plain = plain_transfers(a, maxsel);
         /* N is "defined" whenever the caller passes it (src/SimInf.c:302-305),
          * even if no event shifts. */
@@ -1880,7 +1882,7 @@ static cudaError_t launch_streamed(siminf_gpu_plan *p, DevState s, cudaStream_t 
             }
             /* E and N up to the largest select and shift seen so far */
             if (msel > p->max_select && a->jcE) {
-                if (upload_E(p->s, a, msel, p->owned, st)) {
+                if (upload_E(p, a, msel, st)) {
                     e = cudaErrorMemoryAllocation;
                     break;
                 }
@@ -2406,7 +2408,7 @@ static cudaError_t launch_streamed_dev(siminf_gpu_plan *p, DevState s, cudaStrea
         }
         /* E and N up to the largest select and shift seen so far */
         if (pl.ch.max_select > p->max_select && a->jcE) {
-            if (upload_E(p->s, a, pl.ch.max_select, p->owned, st)) {
+            if (upload_E(p, a, pl.ch.max_select, st)) {
                 e = cudaErrorMemoryAllocation;
                 break;
             }

@@ -7,6 +7,7 @@
 #define SIMINF_CAPI_INTERNAL_H
 
 #include <memory>
+#include <list>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -86,6 +87,8 @@ struct siminf_gpu_plan {
     int nsel = 0;
     int max_select = 0, max_shift = 0;  /* largest select / shift of any event */
     bool e2_plain = true;               /* most transfers are e2_apply's own (plain_transfers) */
+    std::list<std::vector<uint32_t>> ecols; /* sources of the copies to DevState::ecol, the
+                                             * latest last; a copy may outlast its call */
     std::vector<long long> e2_day_off, e2_lo, e2_hi;
     std::vector<std::vector<long long>> day_waves;
     /* Streamed runs: the waves are planned on host threads while the GPU
