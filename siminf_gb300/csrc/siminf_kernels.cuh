@@ -3321,12 +3321,12 @@ static inline unsigned blocks_for(long long n, int threads)
 
 static inline int sm_count()
 {
-    static int n = 0;
-    if (!n) {
-        int dev = 0;
+    static const int n = [] {           /* once, whichever thread comes first */
+        int dev = 0, count = 1;
         cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    }
+        cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+        return count;
+    }();
     return n;
 }
 
@@ -3466,12 +3466,11 @@ struct Launch {
     template <bool WIDE>
     static int aem_resident_blocks()
     {
-        static int blocks = 0;
-        if (!blocks) {
+        static const int blocks = [] {
             int per = 0;
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_aem_day<M, WIDE>, SSA_BLOCK, 0);
-            blocks = sm_count() * (per > 0 ? per : 1);
-        }
+            return sm_count() * (per > 0 ? per : 1);
+        }();
         return blocks;
     }
     template <bool WIDE>
