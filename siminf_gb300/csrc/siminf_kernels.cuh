@@ -5,14 +5,18 @@
  * from generated C code (siminf_gb300/devmodel.py) instantiates them in a
  * library of its own, with the same launcher table.
  *
- * One thread owns one (replicate, node) pair g for the node phases:
- *   k_init       rate initialisation      src/solvers/SimInf_solver_ssm.c:96-117
- *   k_ssa_e1     direct-method SSA up to the next unit of time
+ * The phases of a (replicate, node) pair g and their kernels:
+ *   k_init       rate initialisation, a thread a node
+ *                                          src/solvers/SimInf_solver_ssm.c:96-117
+ *   k_ssa_e1     direct-method SSA up to the next unit of time, a thread or,
+ *                for heavy nodes, a group of 8, 16 or 32 lanes a node
  *                                          src/solvers/SimInf_solver_ssm.c:144-235
  *                followed by the node's E1 events of the day
  *                                          src/solvers/SimInf_solver.c:658-822
+ *   k_quick      the nodes whose day has no transition, ahead of k_ssa_e1
  *   k_e2_wave    one conflict-free wavefront of external transfers
  *                                          src/solvers/SimInf_solver.c:824-902
+ *   k_e2_tail    a day's last wavefronts, in order, by one cluster
  *   k_pts_store  post time step, rate refresh, U/V store
  *                                          src/solvers/SimInf_solver_ssm.c:262-334
  *   k_horizon    all days of one node in one thread, for schedules without
@@ -149,7 +153,7 @@ __device__ __forceinline__ void add_fired(const DevState &s, unsigned long long 
 /*    once per rate update, so choosing the transition is NT-1          */
 /*    independent comparisons instead of a dependent add/compare chain; */
 /*  - divisions, comparisons and int->double conversions run on the     */
-/*    integer pipes (si_div, si_dge/si_dgt, si_i2d): same bits, and a   */
+/*    integer pipes (si_div, si_dge_num, si_i2d): same bits, and a      */
 /*    rate's division by a population count reuses its prepared         */
 /*    reciprocal (si_div_cached).                                       */
 /* Draw i of the node's stream is word i & 3 of Philox block i >> 2; a  */
@@ -597,8 +601,8 @@ __device__ __forceinline__ bool ssa_step_in_order(SsaLane<M> &ln, const si_rng &
 {
     constexpr int NC = M::NC, NT = M::NT;
     const double tn = ln.tau + ln.t;
-    /* the hardware FP64 comparisons of the chain (IEEE, false on NaN, as
-     * si_dge/si_dgt): one instruction each, ~3% off a transition's latency */
+    /* the hardware FP64 comparisons of the chain (false on NaN): one
+     * instruction each, ~3% off a transition's latency */
     if (tn >= next) {
         ln.t = next;
         ln.c += 1;                            /* the waiting time's draw was used */
@@ -2388,10 +2392,11 @@ __global__ void __launch_bounds__(256) k_pts_store(DevState s, int day, double t
 }
 
 /* ------------------------------------------------------------------ */
-/* All-events method (src/solvers/SimInf_solver_aem.c), one thread per   */
-/* node.  Transition j of node g draws from its own stream, keyed (seed, */
-/* AEM_SID | (g * Nt + j)); the next event is the smallest event time,   */
-/* the lowest transition among equal times.                              */
+/* All-events method (src/solvers/SimInf_solver_aem.c), a lane for each  */
+/* transition of a node during its day (k_aem_day), a thread a node at   */
+/* its start and end.  Transition j of node g draws from its own stream, */
+/* keyed (seed, AEM_SID | (g * Nt + j)); the next event is the smallest  */
+/* event time, the lowest transition among equal times.                  */
 /* ------------------------------------------------------------------ */
 #define AEM_SID (1ULL << 63)
 

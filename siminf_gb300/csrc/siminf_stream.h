@@ -593,24 +593,6 @@ SI_HD int si_isnan_bits(uint64_t b)
     return (b << 1) > 0xFFE0000000000000ULL;
 }
 
-/* a > b with IEEE semantics (false when either is NaN). */
-SI_HD int si_dgt(double a, double b)
-{
-    const uint64_t A = si_double_bits(a), B = si_double_bits(b);
-    if (si_isnan_bits(A) || si_isnan_bits(B))
-        return 0;
-    return si_dkey(A) > si_dkey(B);
-}
-
-/* a >= b with IEEE semantics (false when either is NaN). */
-SI_HD int si_dge(double a, double b)
-{
-    const uint64_t A = si_double_bits(a), B = si_double_bits(b);
-    if (si_isnan_bits(A) || si_isnan_bits(B))
-        return 0;
-    return si_dkey(A) >= si_dkey(B);
-}
-
 /* (double) x for a 32-bit integer, exact, from integer bits: the leading
  * one moves to bit 31 and then onto the exponent's lowest bit. */
 SI_HD double si_i2d(int32_t x)
