@@ -57,9 +57,10 @@ UNIT = "node-days/s"
 ALGO_BYTES_PER_NODE_DAY = 16 + 0.504 * 36
 # DRAM traffic of one k_ssa_e1 launch (dram__bytes_read.sum +
 # dram__bytes_write.sum) measured by ncu on this workload at its full node
-# count (10^6 nodes, day 110 of a 120-day run: 93.3 MB read, 10.6 MB
-# written), per node; another node count moves that much per node.
-SSA_TRAFFIC_BYTES_PER_NODE = (93.299968e6 + 10.620928e6) / 1_000_000
+# count with two-pass days (10^6 nodes, day 110 of a 120-day run: 27.8 MB
+# read, 0.5 MB written: the nodes with a transition that day), per node;
+# another node count moves that much per node.
+SSA_TRAFFIC_BYTES_PER_NODE = (27.784192e6 + 0.546560e6) / 1_000_000
 
 
 def parse():

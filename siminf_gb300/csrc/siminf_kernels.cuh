@@ -1792,8 +1792,8 @@ __global__ void __launch_bounds__(256) k_quick(DevState s, int day, double tt, d
  * transitions instead of waiting for the warp's busiest node.
  * Bound: the busiest node's chain, then issue slots and the FP64 pipe.
  * SEIR of 10^6 nodes, 240 days (256,149 steps of the busiest nodes): 501 ms
- * one lane a node, 85.8 with groups and serial sums, 49.6 with the sums as
- * prefix sums of whole numbers; 10,000 nodes x 365 days 136, 22.0, 14.8. */
+ * one lane a node, 85.8 with groups and serial sums, 42.1 with the sums as
+ * prefix sums of whole numbers; 10,000 nodes x 365 days 136, 22.0, 13.0. */
 template <class M, int MINB>
 __global__ void __launch_bounds__(SSA_BLOCK, MINB) k_ssa_e1(DevState s, int day, double tt,
                                                          double next)
@@ -2214,7 +2214,9 @@ __device__ __forceinline__ void cluster_barrier()
  * wave that fills the cluster more than twice is better off on the whole
  * chip.  With e2_apply's common path and draws in step, a day's transfers of
  * SEIR, 10,000 nodes (9.7 waves): 79 us in three launches with a tail of one
- * block, 47 in one launch; 10^6 nodes (15 waves): 187 us, then 138. */
+ * block, 44 in one launch; 10^6 nodes (15 waves): 187 us, then 130.  Waves of
+ * transfers off that path come here in a block's size only
+ * (launch_day_waves). */
 template <class M>
 __global__ void __launch_bounds__(E2_TAIL_BLOCK, 1) k_e2_tail(DevState s, const E2Rec *ev,
                                                            E2Tail tail, int day, double tt)
@@ -2557,7 +2559,7 @@ struct AemLanes {
  * each refresh their own rate and time, side by side: one division a step
  * where one lane did NT of them one after the other.  Bound: the busiest
  * node's chain.  SEIR, 100,000 nodes x 120 days: 50.3 ms with a lane a node,
- * 26.3 with four.
+ * 23.1 with four.
  * With WIDE, for many nodes a group (Launch::aem_day), a warp looks through
  * the ordinary part 32 nodes at a time, a lane a node: one whose event times
  * all pass the day's end, and without an E1 event, is done, and the groups
